@@ -62,57 +62,238 @@ __global__ void k_validate(const int* __restrict__ rowptr, const int* __restrict
     }
 }
 
-// Persistent sync-free level computation over natural-order chunks: warp
-// task t covers rows [32t, 32t+32) and computes them one after another, all
-// 32 lanes striding a row's columns.  Natural order is topological, so a
-// dependency inside the chunk was computed by this warp a moment ago and is
-// read from the warp's shared-memory ring; a dependency outside is polled
-// warp-convergently (level 0 = not yet written).  Row metadata of the whole
-// chunk is loaded up front, one row per lane.
-// With a task table (task_r0 != null), task t covers rows [task_r0[t],
-// task_r0[t] + task_cnt[t]) instead (at most 32 consecutive rows); any
-// order in which every row's dependencies lie in earlier tasks or earlier in
-// its own task is deadlock-free.
-__global__ void __launch_bounds__(256) k_levels(const int* __restrict__ rowptr, const int* __restrict__ col, int n,
-                                                int* level, int* nlevs, DevStatus* st, unsigned long long budget,
-                                                const int* __restrict__ task_r0, const int* __restrict__ task_cnt,
-                                                long long ntask)
+// Persistent sync-free level computation over natural-order groups, one
+// thread per row.  CTA g takes the groups g, g + G, ...: kLvGroup consecutive
+// rows (or, with a task table, the rows [task_r0[t], task_r0[t] +
+// task_cnt[t]); any order in which every row's dependencies lie in earlier
+// tasks or earlier in its own is deadlock-free).  The group's levels live in
+// shared memory (0 = not yet known), so a dependency inside the group is a
+// shared-memory poll; others are polled in global memory.
+//
+// Every lane walks its own row and publishes as soon as the row is done: a
+// warp that holds the end of one grid line and the start of the next must
+// not make the second wait for the first (solving a warp's rows in order did,
+// and strung all lines of a grid behind one another: 322 ms on a 1023 x 1025
+// grid).  Columns inside the row's own warp are not polled.  Where they are
+// the row before only (stencils), a max-plus prefix scan over the lanes closes
+// the warp, the level of the row before the warp entering last, so a grid
+// line costs one hop per warp and not 32 dependent steps.  Otherwise one pass
+// over the lanes that are read, in order, hands each finished level to the
+// lanes that read it (about 45 cycles a lane read, against 600 for a poll
+// round through shared memory), once all rows' outside columns are known or
+// when some are long in coming.
+//
+// Before it looks at all its columns a warp waits for one word: the smallest,
+// over its rows without a column inside the warp, of the row's largest
+// column.  The warp's first finished row is one of those, and thousands of
+// warps that wait far from the front then cost one L2 sector a poll each.
+//
+// Bound: hops.  A value written by one SM is seen by another 707 cycles later
+// (measured, B200), a line costs about 1,700.  Kernel times before and after:
+// 1023 x 1025 grid with holes 322 -> 2.0 ms, 2048 x 2048 grid 2.7 -> 1.9 ms,
+// 101 x 90 x 97 grid 431 -> 0.26 ms, banded n = 1e5 (8 in 256) 44.7 -> 4.0 ms,
+// banded n = 3e5 (4-8 in 16) 132 -> 15.7 ms, Zipf n = 2e6 42 -> 1.5 ms, dense
+// 32-row blocks n = 5e5 58 -> 48 us.
+constexpr int kLvStall = 16;  // polls without an answer after which a warp looks for rows that can do without
+
+template <int U>
+__global__ void __launch_bounds__(kLvGroup) k_levels(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                     int n, int* level, int* nlevs, DevStatus* st,
+                                                     unsigned long long budget, const int* __restrict__ task_r0,
+                                                     const int* __restrict__ task_cnt, long long ntasks)
 {
-    __shared__ int ring[8][32];
-    const int lane = threadIdx.x & 31;
-    int* my = ring[threadIdx.x >> 5];
-    const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long ntasks = task_r0 ? ntask : ((long long)n + 31) / 32;
+    __shared__ volatile int lv[kLvGroup];
+    __shared__ int abort_flag;
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+    const unsigned upto = FULL >> (31 - lane);  // lanes 0..lane
     int my_max = 0;
-    for (long long t = gw; t < ntasks; t += nw) {
-        const int r0 = task_r0 ? __ldg(task_r0 + t) : (int)(t * 32);
-        const int cnt = task_r0 ? __ldg(task_cnt + t) : min(32, n - r0);
-        int ms = 0, me = 0;
-        if (lane < cnt) {
-            ms = __ldg(rowptr + r0 + lane);
-            me = __ldg(rowptr + r0 + lane + 1) - 1;
+    if (tid == 0) abort_flag = 0;
+    for (long long t = blockIdx.x; t < ntasks; t += gridDim.x) {
+        const int R0 = task_r0 ? __ldg(task_r0 + t) : (int)(t * kLvGroup);
+        const int cnt = task_r0 ? __ldg(task_cnt + t) : min(kLvGroup, n - R0);
+        const int r = R0 + tid, w0 = R0 + wib * 32;
+        const bool act = tid < cnt;
+        lv[tid] = 0;
+        int p = 0, e = 0;
+        if (act) {
+            p = __ldg(rowptr + r);
+            e = __ldg(rowptr + r + 1) - 1;
         }
-        for (int j = 0; j < cnt; j++) {
-            const int s = __shfl_sync(0xffffffffu, ms, j), e = __shfl_sync(0xffffffffu, me, j);
-            int m = 0;
-            for (int p = s + lane; __any_sync(0xffffffffu, p < e); p += 32) {
-                const bool have = p < e;
-                const int c = have ? __ldg(col + p) : 0;
-                const bool local = have && c >= r0;
-                int lv = local ? my[c - r0] : 0;
-                if (!warp_wait<false, int>(have && !local, c, level, nullptr, lv, st, budget, 0u, r0 + j)) return;
-                if (have) m = max(m, lv);
+        int c[U], nb = 0, far = -1;
+        unsigned pend = 0;    // columns of the batch outside the warp, not known yet
+        unsigned inmask = 0;  // lanes of this warp the row reads and has not got yet
+        auto batch = [&]() {
+            nb = min(U, e - p);
+            pend = 0;
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                c[u] = -1;
+                if (u < nb) {
+                    c[u] = __ldg(col + p + u);
+                    if (c[u] >= w0) inmask |= 1u << (c[u] - w0);
+                    else pend |= 1u << u;
+                }
             }
-            m = __reduce_max_sync(0xffffffffu, m);
-            if (lane == 0) {
-                my[j] = m + 1;
-                st_relaxed(level + r0 + j, m + 1);
+        };
+        batch();
+        const bool sub = lane > 0 && (inmask >> (lane - 1)) & 1u;
+        // closed by the scan: no lane holds more than U columns, and none inside the warp but the row before
+        const bool chain = __all_sync(FULL, e - p <= U && inmask == (sub ? 1u << (lane - 1) : 0u));
+        unsigned cinbit = 0;  // chain: the column of lane 0 that is the row before the warp
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (pend >> u & 1u) {
+                if (chain && lane == 0 && c[u] == w0 - 1) cinbit = 1u << u;
+                else far = max(far, c[u]);
             }
-            my_max = max(my_max, m + 1);
-            __syncwarp();
+        const bool cin = __shfl_sync(FULL, cinbit, 0) != 0;
+        int word = __reduce_min_sync(FULL, act && inmask == 0 ? (cinbit ? w0 - 1 : far) : 0x7fffffff);
+        if (cin && word == w0 - 1) {
+            // the row before the warp comes last in a scan: the line above is awaited first
+            const int above = __reduce_min_sync(FULL, far >= 0 ? far : 0x7fffffff);
+            if (above != 0x7fffffff) word = above;
         }
+        __syncthreads();  // lv is filled
+        bool fail = false;
+        unsigned it = 0, seen = 0;
+        unsigned long long t0 = 0;
+        if (word >= 0 && word != 0x7fffffff)
+            while ((word >= R0 ? lv[word - R0] : ld_relaxed(level + word)) == 0)
+                if ((++it & 63u) == 0 && give_up(t0, st, budget, w0)) {
+                    fail = true;
+                    break;
+                }
+        bool done = !act, ready = !act;  // ready: all columns outside the warp are known
+        int m = 0, A = 0, vin = 0;
+        // segments of rows linked to the row before: their first lanes, and this lane's
+        const unsigned S = __ballot_sync(FULL, !sub) | 1u;
+        const int start = 31 - __clz(S & upto);
+        const unsigned need = upto & (FULL << start);
+        bool all = true;  // poll every pending column
+        bool stalled = false;
+        while (!fail) {
+            if (all) {
+                int v[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    v[u] = 0;
+                    if ((pend >> u & 1u) && c[u] < R0) v[u] = ld_relaxed(level + c[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if ((pend >> u & 1u) && c[u] >= R0) v[u] = lv[c[u] - R0];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (v[u] != 0) {
+                        pend &= ~(1u << u);
+                        if (cinbit >> u & 1u) vin = v[u];
+                        else m = max(m, v[u]);
+                    }
+            }
+            bool again = false;
+            if (!ready && (pend & ~cinbit) == 0) {
+                p += nb;
+                if (p < e) {
+                    batch();
+                    again = true;
+                } else {
+                    ready = true;
+                }
+            }
+            const unsigned R = __ballot_sync(FULL, ready);
+            if (chain) {
+                if (R != seen) {
+                    seen = R;
+                    A = m + 1;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const int Ap = __shfl_up_sync(FULL, A, d);
+                        if (lane - d >= start) A = max(A, Ap + d);
+                    }
+                }
+                const int in = __shfl_sync(FULL, vin, 0);
+                const bool hang = start == 0 && cin;  // the segment hangs on the row before the warp
+                if (!done && (R & need) == need && (!hang || in != 0)) {
+                    const int l = hang ? max(A, in + lane + 1) : A;
+                    lv[tid] = l;
+                    st_relaxed(level + r, l);
+                    my_max = max(my_max, l);
+                    done = true;
+                }
+            } else if (R == FULL) {
+                // every row's outside columns are known: one pass in order, each lane final by its turn
+                int l = m + 1;
+                const unsigned T = __reduce_or_sync(FULL, inmask);
+#pragma unroll
+                for (int q = 0; q < 31; q++)
+                    if (T >> q & 1u) {
+                        const int lq = __shfl_sync(FULL, l, q);
+                        if (inmask >> q & 1u) l = max(l, lq + 1);
+                    }
+                if (!done) {
+                    lv[tid] = l;
+                    st_relaxed(level + r, l);
+                    my_max = max(my_max, l);
+                }
+                break;
+            } else {
+                if (stalled && R != seen) {
+                    // some columns are long in coming: the rows that can be done without them are
+                    seen = R;
+                    for (unsigned T = __reduce_or_sync(FULL, ready ? inmask : 0u) & R; T; T &= T - 1) {
+                        const int q = __ffs(T) - 1;
+                        const int lq = __shfl_sync(FULL, inmask == 0 ? m + 1 : 0, q);
+                        if (lq != 0 && ready && (inmask >> q & 1u)) {
+                            m = max(m, lq);
+                            inmask &= ~(1u << q);
+                        }
+                    }
+                }
+                if (ready && inmask == 0 && !done) {
+                    lv[tid] = m + 1;
+                    st_relaxed(level + r, m + 1);
+                    my_max = max(my_max, m + 1);
+                    done = true;
+                }
+            }
+            if (!__any_sync(FULL, !done)) break;
+            all = __any_sync(FULL, again);
+            stalled = false;
+            if (!all) {
+                // nothing to do before some lane's last pending column is known: in natural
+                // order the others mostly come before it
+                const int hi = 31 - __clz(pend);
+                int cc = -1, v = 0;
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (hi == u) cc = c[u];
+                for (int k = 0;; k++) {
+                    if (cc >= R0) v = lv[cc - R0];
+                    else if (cc >= 0) v = ld_relaxed(level + cc);
+                    if (__any_sync(FULL, v != 0)) break;
+                    if (k == kLvStall && !chain && R != seen) {
+                        stalled = true;
+                        break;
+                    }
+                    if ((++it & 63u) == 0 && give_up(t0, st, budget, w0)) {
+                        fail = true;
+                        break;
+                    }
+                }
+                if (v != 0) {
+                    pend &= ~(1u << hi);
+                    if (cinbit >> hi & 1u) vin = v;
+                    else m = max(m, v);
+                }
+                all = __any_sync(FULL, v != 0 && pend != 0);
+            }
+        }
+        if (fail) abort_flag = 1;
+        __syncthreads();  // the group's levels are read no more
+        if (abort_flag) return;
     }
+    my_max = __reduce_max_sync(FULL, my_max);
     if (lane == 0 && my_max > 0) atomicMax(nlevs, my_max);
 }
 
@@ -262,10 +443,10 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     // 1. levels
     int nlevs = 0;
     if (n > 0) {
-        // one 32-row chunk per warp, 8 warps per block
-        const long long nt = tasks ? tasks->n : ((long long)n + 31) / 32;
-        ACHK(launch_persistent(k_levels, 256, 0, (nt + 7) / 8, s, L->ia, L->ja, n, rec->d_levels, d_nlevs,
-                               c->d_status, wait_budget_ns(), tasks ? tasks->r0 : (const int*)nullptr,
+        const long long nt = tasks ? tasks->n : ((long long)n + kLvGroup - 1) / kLvGroup;
+        // columns per lane and poll round: 4 covers a stencil's row at once
+        auto kern = (long long)nnz - n <= 4LL * n ? k_levels<4> : k_levels<8>;
+        ACHK(launch_persistent(kern, kLvGroup, 0, nt, s, L->ia, L->ja, n, rec->d_levels, d_nlevs, c->d_status, wait_budget_ns(), tasks ? tasks->r0 : (const int*)nullptr,
                                tasks ? tasks->cnt : (const int*)nullptr, nt));
         ACHK(cudaMemcpyAsync(&nlevs, d_nlevs, sizeof(int), cudaMemcpyDeviceToHost, s));
         int st = sync_status(s);

@@ -1155,20 +1155,20 @@ int sptrsv_batch_create(int nsys, const sp_mat_t* mats, const int* nrhs, sptrsv_
         U.nr = U.nc = (int)n;
         U.nnz = (int)nnz;
         // 2. levels of the union (validates every system's CSR too).  The level
-        // kernel takes 32-row chunks system by system in order of their index
+        // kernel takes groups of rows system by system in order of their index
         // inside their system, so the dependency chains of all systems advance
-        // together; in natural order a warp's chunk deep in one system's chain
-        // holds up its later chunks of other systems (creating the 512-system
-        // banded batch of up to 200,000 rows per system took 8.1 s, now 0.24 s).
+        // together; in natural order a CTA's group deep in one system's chain
+        // holds up its later groups of other systems (creating the 512-system
+        // banded batch of up to 200,000 rows per system took 8.1 s, then 0.24 s).
         {
             int maxc = 0;
-            for (int k = 0; k < nsys; k++) maxc = std::max(maxc, (mats[k].nr + 31) / 32);
+            for (int k = 0; k < nsys; k++) maxc = std::max(maxc, (mats[k].nr + kLvGroup - 1) / kLvGroup);
             std::vector<int> tr0, tcnt;
             for (int c = 0; c < maxc; c++)
                 for (int k = 0; k < nsys; k++)
-                    if (c * 32 < mats[k].nr) {
-                        tr0.push_back(row0[k] + c * 32);
-                        tcnt.push_back(std::min(32, mats[k].nr - c * 32));
+                    if (c * kLvGroup < mats[k].nr) {
+                        tr0.push_back(row0[k] + c * kLvGroup);
+                        tcnt.push_back(std::min(kLvGroup, mats[k].nr - c * kLvGroup));
                     }
             int *d_tr0 = nullptr, *d_tcnt = nullptr;
             cudaError_t ce = dalloc(&d_tr0, (long long)tr0.size());

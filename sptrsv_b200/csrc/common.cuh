@@ -103,6 +103,25 @@ __device__ __forceinline__ void report(DevStatus* st, int code, int row)
     if (atomicCAS(&st->code, 0, code) == 0) st->row = row;
 }
 
+// The bound of a warp's wait loop, called by all 32 lanes every few polls:
+// true (warp-uniform) when the loop has run for budget nanoseconds since its
+// first check (*t0, 0 before) or another warp reported an error.
+__device__ __forceinline__ bool give_up(unsigned long long& t0, DevStatus* st, unsigned long long budget, int row)
+{
+    int stop = 0;
+    if ((threadIdx.x & 31) == 0) {
+        const unsigned long long now = global_ns();
+        if (t0 == 0) t0 = now;
+        if (ld_relaxed(&st->code) != 0) {
+            stop = 1;
+        } else if (now - t0 > budget) {
+            report(st, SPTRSV_ERR_TIMEOUT, row);
+            stop = 1;
+        }
+    }
+    return __shfl_sync(0xffffffffu, stop, 0) != 0;
+}
+
 // Spin until *p is no longer the sentinel.  Returns false if the wait ran out
 // or another warp reported an error (the caller then leaves the kernel).
 // After 8 failed polls the loop sleeps `backoff_ns` between polls (0: spin),

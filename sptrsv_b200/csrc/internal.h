@@ -189,8 +189,10 @@ struct AnalysisRec {
 };
 void register_analysis(const int* key, AnalysisRec* rec);
 
-// Task order for the level kernel: task t covers the cnt[t] <= 32 rows from
-// r0[t]; null keeps consecutive 32-row chunks in natural order.
+// Rows of one task of the level kernel (one CTA, one thread per row).
+constexpr int kLvGroup = 256;
+// Task order for the level kernel: task t covers the cnt[t] <= kLvGroup rows
+// from r0[t]; null keeps consecutive groups in natural order.
 struct LevelTasks {
     const int* r0;
     const int* cnt;
