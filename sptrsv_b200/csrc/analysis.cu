@@ -363,12 +363,11 @@ __global__ void k_inverse(const int* __restrict__ perm, int n, int* __restrict__
 }  // namespace
 
 // Checks a device CSR; returns 0, SPTRSV_ERR_INVALID_CSR (with *bad_row) or a CUDA error code.
-int validate_csr_device(const int* rowptr, const int* col, int n, int nnz, cudaStream_t s, int* bad_row)
+// d_res: two device ints of scratch.
+int validate_csr_device(const int* rowptr, const int* col, int n, int nnz, int* d_res, cudaStream_t s, int* bad_row)
 {
     *bad_row = -1;
     if (n <= 0) return 0;
-    int* d_res = nullptr;
-    SPT_CUDA(cudaMalloc((void**)&d_res, 2 * sizeof(int)));
     int h[2] = {0, 0x7fffffff};
     cudaError_t e = cudaMemcpyAsync(d_res, h, sizeof(h), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
@@ -377,7 +376,6 @@ int validate_csr_device(const int* rowptr, const int* col, int n, int nnz, cudaS
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(h, d_res, sizeof(h), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    cudaFree(d_res);
     if (e != cudaSuccess) return cuda_fail(e, "validate_csr_device");
     if (h[0]) {
         *bad_row = h[1];
@@ -398,31 +396,17 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     cudaStream_t s = 0;
     const int nnz = L->nnz;
 
-    // 0. validation (the status block must be clean before the bounded waits)
-    {
-        int e = sync_status(s);
-        if (e) return e;
-        int bad = -1;
-        e = validate_csr_device(L->ia, L->ja, n, nnz, s, &bad);
-        if (e == SPTRSV_ERR_INVALID_CSR)
-            return set_error(e, "analysis: row %d is not lower-triangular CSR with sorted columns and the diagonal last",
-                             bad);
-        if (e) return e;
-    }
-
+    // A device allocation and its release cost about 0.1 ms each, whatever
+    // their size, so the arrays share four: what n alone sizes, scratch, what
+    // the level count sizes, and the warp map.
     AnalysisRec* rec = new AnalysisRec();
     rec->device = c->device;
     rec->n = n;
     rec->nnz = nnz;
-    int *d_key = nullptr, *d_key2 = nullptr, *d_val2 = nullptr, *d_scr = nullptr, *d_nlevs = nullptr;
-    int *d_iorder = nullptr, *d_rowctr = nullptr, *d_levsz = nullptr, *d_inv = nullptr;
-    int *d_wpk = nullptr, *d_rowoff = nullptr;
+    int* scratch = nullptr;
     auto fail = [&](int code) {
-        cudaFree(d_key); cudaFree(d_key2); cudaFree(d_val2); cudaFree(d_scr); cudaFree(d_nlevs);
-        cudaFree(d_iorder); cudaFree(d_rowctr); cudaFree(d_levsz); cudaFree(d_inv);
-        cudaFree(d_wpk); cudaFree(d_rowoff);
-        cudaFree(rec->d_levels); cudaFree(rec->d_counts); cudaFree(rec->d_ibase); cudaFree(rec->d_ivect);
-        cudaFree(rec->d_wlev);
+        cudaFree(scratch);
+        for (int* q : rec->slab) cudaFree(q);
         delete rec;
         return code;
     };
@@ -431,11 +415,29 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
         cudaError_t e_ = (call);                                \
         if (e_ != cudaSuccess) return fail(cuda_fail(e_, #call)); \
     } while (0)
+    auto part = [](long long ints) { return (ints + 63) / 64 * 64; };  // 256-byte aligned
+    const long long pn = part(n);
+    ACHK(dalloc(&rec->slab[0], 3 * pn + 64));
+    int* d_rowctr = rec->slab[0];
+    rec->d_levels = d_rowctr + 64;
+    int *d_iorder = rec->d_levels + pn, *d_inv = d_iorder + pn;
+    const long long scr = radix_scratch_ints(n), keys = 3 * pn;
+    ACHK(dalloc(&scratch, keys + part(scr) + 64));
+    int *d_key = scratch, *d_key2 = d_key + pn, *d_val2 = d_key2 + pn, *d_scr = d_val2 + pn;
+    int* d_nlevs = d_scr + part(scr);
 
-    ACHK(dalloc(&rec->d_levels, n));
-    ACHK(dalloc(&d_nlevs, 1));
-    ACHK(dalloc(&d_iorder, n));
-    ACHK(dalloc(&d_rowctr, 1));
+    // 0. validation (the status block must be clean before the bounded waits)
+    {
+        int e = sync_status(s);
+        if (e) return fail(e);
+        int bad = -1;
+        e = validate_csr_device(L->ia, L->ja, n, nnz, d_nlevs + 2, s, &bad);
+        if (e) fail(e);
+        if (e == SPTRSV_ERR_INVALID_CSR)
+            return set_error(e, "analysis: row %d is not lower-triangular CSR with sorted columns and the diagonal last",
+                             bad);
+        if (e) return e;
+    }
     ACHK(cudaMemsetAsync(rec->d_levels, 0, sizeof(int) * (size_t)(n > 0 ? n : 1), s));
     ACHK(cudaMemsetAsync(d_nlevs, 0, sizeof(int), s));
     ACHK(cudaMemsetAsync(d_rowctr, 0, sizeof(int), s));
@@ -456,36 +458,40 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     const long long K = 7LL * nlevs;
 
     // 2-3. keys, counts, stable sort
-    ACHK(dalloc(&rec->d_counts, K + 1));
+    ACHK(dalloc(&rec->slab[1], part(K + 1) + part(nlevs)));
+    rec->d_counts = rec->slab[1];
+    int* d_levsz = rec->d_counts + part(K + 1);
     ACHK(cudaMemsetAsync(rec->d_counts, 0, sizeof(int) * (size_t)(K + 1), s));
-    ACHK(dalloc(&d_key, n));
-    ACHK(dalloc(&d_key2, n));
-    ACHK(dalloc(&d_val2, n));
-    long long scr = radix_scratch_ints(n);
-    long long scr2 = scan_scratch_ints(K + 1);
-    ACHK(dalloc(&d_scr, scr > scr2 ? scr : scr2));
     if (n > 0) {
         k_keys<<<grid_for(n, 256), 256, 0, s>>>(L->ia, rec->d_levels, n, d_key, d_iorder, rec->d_counts);
         ACHK(cudaGetLastError());
         ACHK(radix_sort_pairs(d_key, d_iorder, d_key2, d_val2, n, (int)(K - 1), d_scr, s));
     }
 
-    // 4. multirow warp map (always built; exposed in info for MULTIROW/ALL)
-    ACHK(dalloc(&d_wpk, K + 1));
-    ACHK(dalloc(&d_rowoff, K + 1));
+    // 4. multirow warp map (always built; exposed in info for MULTIROW/ALL),
+    // its scratch where the sort's keys were unless there are more keys than rows
+    const long long map_scr = 2 * part(K + 1) + part(scan_scratch_ints(K + 1));
+    if (map_scr > keys) {
+        cudaFree(scratch);
+        scratch = nullptr;
+        ACHK(dalloc(&scratch, map_scr));
+    }
+    int *d_wpk = scratch, *d_rowoff = d_wpk + part(K + 1), *d_scr2 = d_rowoff + part(K + 1);
     int n_warps = 0;
     if (K > 0) {
         k_warps_per_key<<<grid_for(K + 1, 256), 256, 0, s>>>(rec->d_counts, (int)K, d_wpk);
         ACHK(cudaGetLastError());
-        ACHK(scan_exclusive(d_wpk, d_wpk, K + 1, d_scr, s));
-        ACHK(scan_exclusive(rec->d_counts, d_rowoff, K + 1, d_scr, s));
+        ACHK(scan_exclusive(d_wpk, d_wpk, K + 1, d_scr2, s));
+        ACHK(scan_exclusive(rec->d_counts, d_rowoff, K + 1, d_scr2, s));
         ACHK(cudaMemcpyAsync(&n_warps, d_wpk + K, sizeof(int), cudaMemcpyDeviceToHost, s));
         ACHK(cudaStreamSynchronize(s));
     }
     rec->n_warps = n_warps;
-    ACHK(dalloc(&rec->d_ibase, (long long)n_warps + 1));
-    ACHK(dalloc(&rec->d_ivect, n_warps));
-    ACHK(dalloc(&rec->d_wlev, n_warps));
+    const long long pw = part((long long)n_warps + 1);
+    ACHK(dalloc(&rec->slab[2], 3 * pw));
+    rec->d_ibase = rec->slab[2];
+    rec->d_ivect = rec->d_ibase + pw;
+    rec->d_wlev = rec->d_ivect + pw;
     if (n_warps > 0) {
         k_warp_map<<<grid_for(n_warps, 256), 256, 0, s>>>(d_wpk, d_rowoff, (int)K, n_warps, n, rec->d_ibase,
                                                            rec->d_ivect, rec->d_wlev);
@@ -495,8 +501,6 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     }
 
     // extras the reference declares but never fills
-    ACHK(dalloc(&d_levsz, nlevs));
-    ACHK(dalloc(&d_inv, n));
     if (nlevs > 0) {
         k_level_sizes<<<grid_for(nlevs, 256), 256, 0, s>>>(rec->d_counts, nlevs, d_levsz);
         ACHK(cudaGetLastError());
@@ -506,13 +510,7 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
         ACHK(cudaGetLastError());
     }
     ACHK(cudaStreamSynchronize(s));
-    cudaFree(d_key);
-    cudaFree(d_key2);
-    cudaFree(d_val2);
-    cudaFree(d_scr);
-    cudaFree(d_nlevs);
-    cudaFree(d_wpk);
-    cudaFree(d_rowoff);
+    cudaFree(scratch);
 #undef ACHK
 
     info->mode = mode;

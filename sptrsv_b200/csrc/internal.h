@@ -183,6 +183,7 @@ struct AnalysisRec {
     int* d_ibase = nullptr;    // [n_warps+1] multirow map (always built)
     int* d_ivect = nullptr;    // [n_warps]
     int* d_wlev = nullptr;     // [n_warps]
+    int* slab[3] = {};         // the allocations that hold these arrays and the info struct's
     bool map_in_info = false;  // map arrays are also referenced by the info struct
     int* tile_tasks[6] = {};   // level-aligned iorder tasks for 32>>j lanes per row
     int tile_ntasks[6] = {};

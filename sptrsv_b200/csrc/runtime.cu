@@ -307,19 +307,15 @@ void free_device_analysis(sp_mat_t* gpu_L, dfr_analysis_info_t* info)
     ::sptrsv::abi_guard_void([&] {
         if (info) {
             AnalysisRec* rec = info->row_ctr ? unregister_analysis(info->row_ctr) : nullptr;
-            cudaFree(info->iorder);
-            cudaFree(info->row_ctr);
-            cudaFree(info->lev_size);
-            cudaFree(info->inv_iorder);
             if (rec) {
-                cudaFree(rec->d_levels);
-                cudaFree(rec->d_counts);
-                cudaFree(rec->d_ibase);
-                cudaFree(rec->d_ivect);
-                cudaFree(rec->d_wlev);
+                for (int* q : rec->slab) cudaFree(q);  // every array of info is part of one of them
                 for (int j = 0; j < 6; j++) cudaFree(rec->tile_tasks[j]);
                 delete rec;
             } else {
+                cudaFree(info->iorder);
+                cudaFree(info->row_ctr);
+                cudaFree(info->lev_size);
+                cudaFree(info->inv_iorder);
                 cudaFree(info->ibase_row);
                 cudaFree(info->ivect_size_warp);
                 cudaFree(info->warp_lev);
