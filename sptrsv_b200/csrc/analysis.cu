@@ -298,12 +298,15 @@ __global__ void __launch_bounds__(kLvGroup) k_levels(const int* __restrict__ row
 }
 
 __global__ void k_keys(const int* __restrict__ rowptr, const int* __restrict__ level, int n, int* __restrict__ key,
-                       int* __restrict__ iota, int* counts)
+                       int* __restrict__ iota, int* counts, int* longer)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int k = 7 * (level[i] - 1) + bucket_of(rowptr[i + 1] - rowptr[i] - 1);
+        const int len = rowptr[i + 1] - rowptr[i] - 1;
+        int k = 7 * (level[i] - 1) + bucket_of(len);
         key[i] = k;
         iota[i] = i;
+        const unsigned over = __ballot_sync(__activemask(), len > 32);
+        if (over && (threadIdx.x & 31) == __ffs(over) - 1) atomicAdd(longer, __popc(over));
         unsigned peers = __match_any_sync(__activemask(), k);
         if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(counts + k, __popc(peers));
     }
@@ -344,13 +347,35 @@ __global__ void k_warp_map(const int* __restrict__ warp_off, const int* __restri
     }
 }
 
-__global__ void k_level_sizes(const int* __restrict__ counts, int nlevs, int* __restrict__ lev_size)
+// Sizes and first positions of the levels, and the statistics that
+// choose_level_cta reads: stats[c] = sum over the levels past the first of
+// ceil(size / (4 << c)) - 1, the steps beyond one of a CTA that takes 4 << c
+// rows of a level at once; stats[8 + b] = rows of bucket b; stats[15] = rows
+// of more than 32 off-diagonals (k_keys).
+__global__ void k_level_sizes(const int* __restrict__ counts, const int* __restrict__ row_off, int nlevs,
+                              int* __restrict__ lev_size, int* __restrict__ lptr, int* stats)
 {
-    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < nlevs; l += gridDim.x * blockDim.x) {
+    __shared__ int acc[16];
+    if (threadIdx.x < 16) acc[threadIdx.x] = 0;
+    __syncthreads();
+    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l <= nlevs; l += gridDim.x * blockDim.x) {
+        lptr[l] = row_off[7 * l];  // row_off[7 * nlevs] = n
+        if (l == nlevs) break;
         int s = 0;
-        for (int b = 0; b < 7; b++) s += counts[7 * l + b];
+        for (int b = 0; b < 7; b++) {
+            const int k = counts[7 * l + b];
+            s += k;
+            if (k) atomicAdd(acc + 8 + b, k);
+        }
         lev_size[l] = s;
+        if (l > 0)
+            for (int c = 0; c < 8; c++) {
+                const int extra = (s - 1) >> (2 + c);
+                if (extra) atomicAdd(acc + c, extra);
+            }
     }
+    __syncthreads();
+    if (threadIdx.x < 16 && acc[threadIdx.x]) atomicAdd(stats + threadIdx.x, acc[threadIdx.x]);
 }
 
 __global__ void k_inverse(const int* __restrict__ perm, int n, int* __restrict__ inv)
@@ -458,12 +483,15 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     const long long K = 7LL * nlevs;
 
     // 2-3. keys, counts, stable sort
-    ACHK(dalloc(&rec->slab[1], part(K + 1) + part(nlevs)));
+    ACHK(dalloc(&rec->slab[1], part(K + 1) + 2 * part((long long)nlevs + 1) + 64));
     rec->d_counts = rec->slab[1];
     int* d_levsz = rec->d_counts + part(K + 1);
+    rec->d_lptr = d_levsz + part((long long)nlevs + 1);
+    int* d_stats = rec->d_lptr + part((long long)nlevs + 1);
     ACHK(cudaMemsetAsync(rec->d_counts, 0, sizeof(int) * (size_t)(K + 1), s));
+    ACHK(cudaMemsetAsync(d_stats, 0, 16 * sizeof(int), s));
     if (n > 0) {
-        k_keys<<<grid_for(n, 256), 256, 0, s>>>(L->ia, rec->d_levels, n, d_key, d_iorder, rec->d_counts);
+        k_keys<<<grid_for(n, 256), 256, 0, s>>>(L->ia, rec->d_levels, n, d_key, d_iorder, rec->d_counts, d_stats + 15);
         ACHK(cudaGetLastError());
         ACHK(radix_sort_pairs(d_key, d_iorder, d_key2, d_val2, n, (int)(K - 1), d_scr, s));
     }
@@ -483,6 +511,10 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
         ACHK(cudaGetLastError());
         ACHK(scan_exclusive(d_wpk, d_wpk, K + 1, d_scr2, s));
         ACHK(scan_exclusive(rec->d_counts, d_rowoff, K + 1, d_scr2, s));
+        k_level_sizes<<<grid_for(nlevs + 1LL, 256), 256, 0, s>>>(rec->d_counts, d_rowoff, nlevs, d_levsz, rec->d_lptr,
+                                                                 d_stats);
+        ACHK(cudaGetLastError());
+        ACHK(cudaMemcpyAsync(rec->stats, d_stats, 16 * sizeof(int), cudaMemcpyDeviceToHost, s));
         ACHK(cudaMemcpyAsync(&n_warps, d_wpk + K, sizeof(int), cudaMemcpyDeviceToHost, s));
         ACHK(cudaStreamSynchronize(s));
     }
@@ -501,10 +533,6 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     }
 
     // extras the reference declares but never fills
-    if (nlevs > 0) {
-        k_level_sizes<<<grid_for(nlevs, 256), 256, 0, s>>>(rec->d_counts, nlevs, d_levsz);
-        ACHK(cudaGetLastError());
-    }
     if (n > 0) {
         k_inverse<<<grid_for(n, 256), 256, 0, s>>>(d_iorder, n, d_inv);
         ACHK(cudaGetLastError());

@@ -183,11 +183,19 @@ struct AnalysisRec {
     int* d_ibase = nullptr;    // [n_warps+1] multirow map (always built)
     int* d_ivect = nullptr;    // [n_warps]
     int* d_wlev = nullptr;     // [n_warps]
+    int* d_lptr = nullptr;     // [nlevs+1] first iorder position of each level
+    int stats[16] = {};        // level widths and row lengths (k_level_sizes)
     int* slab[3] = {};         // the allocations that hold these arrays and the info struct's
     bool map_in_info = false;  // map arrays are also referenced by the info struct
     int* tile_tasks[6] = {};   // level-aligned iorder tasks for 32>>j lanes per row
     int tile_ntasks[6] = {};
 };
+// How one CTA would take a system level by level (level_cta.cuh): kp lanes per
+// row, teams of g warps; kp = 0: the sync-free kernels are the faster ones.
+struct LevelCtaShape {
+    int kp, g;
+};
+LevelCtaShape choose_level_cta(int nlevs, int n, const int* stats, bool level_ordered);
 void register_analysis(const int* key, AnalysisRec* rec);
 
 // Rows of one task of the level kernel (one CTA, one thread per row).

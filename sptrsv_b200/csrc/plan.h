@@ -137,6 +137,8 @@ struct sptrsv_plan_s {
     int* levels = nullptr;       // 1-based level per row
     int* ibase = nullptr;        // multirow map
     int* ivect = nullptr;
+    int* lptr = nullptr;         // [nlevs+1] first position of each level
+    int stats[16] = {};          // level widths and row lengths (AnalysisRec)
     int* ord_tasks[6] = {};      // level-aligned tasks over the level layout, R = 1 << j rows
     int ord_ntasks[6] = {};
     SptLayout clu;               // cluster order (built on demand)

@@ -5,6 +5,7 @@
 #include <cstring>
 
 #include "internal.h"
+#include "level_cta.cuh"
 #include "plan.h"
 #include "solve_kernels.cuh"
 
@@ -68,6 +69,69 @@ int tile_tasks(AnalysisRec* rec, const int* iorder, int lanes, const int** tasks
 
 }  // namespace
 
+// Estimated cycles of a solve by one CTA against the sync-free kernels, both
+// from measurements on B200 (FP64).  One CTA: a level costs 260 cycles with 16
+// teams of one warp, 330, 430 and 850 with 8, 4 and 2 larger teams (n = 2e4
+// in a band of 16, n = 1e5 in 256, n = 5e4 in 1000), and the one SM's load
+// unit 8 cycles a row of a level-ordered copy, 11 of the caller's CSR (a
+// 333 x 277 grid: 367 and 521 us); a step beyond the first of a level, or a
+// level with a row of more than 4 kp entries, 2,600 more.  The sync-free
+// kernels: 1,600 to 1,900 a level whatever its width up to some thousand rows
+// (832, 4095 and 6219 levels).
+LevelCtaShape choose_level_cta(int nlevs, int n, const int* stats, bool level_ordered)
+{
+    static const double kBase[4] = {260, 330, 430, 850};
+    const double extra = 2600, rows = (level_ordered ? 8.0 : 11.0) * n;
+    LevelCtaShape best{0, 0};
+    double best_cost = 0.85 * 1600 * nlevs;
+    for (int j = 0; j < 4; j++) {  // kp = 1 << j lanes hold 4 kp entries of a row
+        double longer = stats[15];
+        if (j < 3)
+            for (int bk = j + 3; bk < 6; bk++) longer += stats[8 + bk];
+        longer = std::min<double>(longer, nlevs);
+        for (int k = 0; k < 4; k++) {  // g = 1 << k: 32 g / kp rows at once
+            const double cost = std::max(kBase[k] * nlevs, rows) + extra * (stats[3 + k - j] + longer);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = {1 << j, 1 << k};
+            }
+        }
+    }
+    return best;
+}
+
+namespace {
+
+constexpr size_t kLevelCtaSmem = 200 * 1024;  // x whole when it fits this, else a ring
+constexpr int kLevelCtaRing = 16384;
+
+template <class M, typename T, typename BT, int OUT, int KP>
+int launch_level_cta_kp(const M& m, const LevelCta& lc, bool ring, int g, const BT* b, T* x, double* x64, cudaStream_t s)
+{
+    auto kern = ring ? k_sptrsv_level_cta<M, T, BT, OUT, KP, true> : k_sptrsv_level_cta<M, T, BT, OUT, KP, false>;
+    const size_t smem = sizeof(T) * ((size_t)lc.slots + 1);
+    if (smem > 32 * 1024) SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<1, 32 * kTeamWarps, smem, s>>>(m, lc, g, b, x, x64);
+    SPT_CUDA(cudaGetLastError());
+    return 0;
+}
+
+template <class M, typename T, typename BT, int OUT>
+int launch_level_cta(const M& m, LevelCtaShape sh, const int* lptr, const int* inv, int nlevs, int n, int divide,
+                     const BT* b, T* x, double* x64, cudaStream_t s)
+{
+    const bool ring = sizeof(T) * ((size_t)n + 1) > kLevelCtaSmem;
+    const LevelCta lc{lptr, inv, nlevs, ring ? kLevelCtaRing : n, divide};
+    switch (sh.kp) {
+    case 1: return launch_level_cta_kp<M, T, BT, OUT, 1>(m, lc, ring, sh.g, b, x, x64, s);
+    case 2: return launch_level_cta_kp<M, T, BT, OUT, 2>(m, lc, ring, sh.g, b, x, x64, s);
+    case 4: return launch_level_cta_kp<M, T, BT, OUT, 4>(m, lc, ring, sh.g, b, x, x64, s);
+    default: return launch_level_cta_kp<M, T, BT, OUT, 8>(m, lc, ring, sh.g, b, x, x64, s);
+    }
+}
+
+}  // namespace
+
 // Reference-named solves over the caller's CSR.  lanes = 0 picks the
 // reference's choice (simple: by nnz/n; order: 32).
 int solve_reference(sp_mat_t* mat, dfr_analysis_info_t* info, const double* b, double* x, int n, MODE mode,
@@ -80,6 +144,17 @@ int solve_reference(sp_mat_t* mat, dfr_analysis_info_t* info, const double* b, d
     if (mode != SIMPLE && (!info || !info->iorder))
         return set_error(SPTRSV_ERR_NOT_ANALYSED, "solve: ORDER/MULTIROW need an analysis");
     if (lanes && !pow2_lanes(lanes)) return set_error(SPTRSV_ERR_INVALID_ARG, "solve: lanes must be 1,2,4,8,16,32");
+    if (mode != SIMPLE) {
+        // few rows per level: one CTA (its result does not depend on `lanes`)
+        AnalysisRec* rec = find_analysis(info->row_ctr);
+        const LevelCtaShape sh = rec && rec->n == n ? choose_level_cta(rec->nlevs, n, rec->stats, false) : LevelCtaShape{0, 0};
+        if (sh.kp) {
+            const NatMat m{mat->ia, mat->ja, mat->a, info->iorder, mat->nnz};
+            int e = launch_level_cta<NatMat, double, double, OUT_X>(m, sh, rec->d_lptr, info->inv_iorder, rec->nlevs, n,
+                                                                    mode == MULTIROW, b, x, nullptr, s);
+            return e ? e : ok();
+        }
+    }
     SPT_CUDA(cudaMemsetAsync(x, 0xFF, sizeof(double) * (size_t)n, s));
     NatMat m{mat->ia, mat->ja, mat->a, mode == SIMPLE ? nullptr : info->iorder};
     auto kern = k_sptrsv<NatMat, double, double, OUT_X>;
@@ -176,7 +251,7 @@ void plan_free_arrays(sptrsv_plan_s* p)
     layout_free(p->clu);
     strip_free(p->strip);
     wave_free(p->wave);
-    cudaFree(p->cptr); cudaFree(p->inv); cudaFree(p->levels); cudaFree(p->ibase); cudaFree(p->ivect);
+    cudaFree(p->cptr); cudaFree(p->inv); cudaFree(p->levels); cudaFree(p->lptr); cudaFree(p->ibase); cudaFree(p->ivect);
     for (int j = 0; j < 6; j++) {
         cudaFree(p->ord_tasks[j]);
         mrhs_free(p->mrhs[j]);
@@ -382,6 +457,18 @@ int plan_launch(sptrsv_plan_s* p, bool f32, const BT* b, T* x, double* x64, int 
     };
     if (sc.variant == SPTRSV_VAR_BAND && nrhs == 1)
         return band_solve(p, f32, b, sizeof(BT) == 4, x, x64, OUT, s);
+    if ((sc.variant == SPTRSV_VAR_ORDER || sc.variant == SPTRSV_VAR_MULTIROW) && nrhs == 1) {
+        const LevelCtaShape sh = choose_level_cta(p->nlevs, n, p->stats, true);
+        if (sh.kp) {
+            const V *val, *dg, *di;
+            layout_vals(p->lev, val, dg, di);
+            const PermMat<V> m{p->lev.ptr, p->lev.rowid, p->lev.col, val, dg, di, nullptr};
+            return launch_level_cta<PermMat<V>, T, BT, OUT>(m, sh, p->lptr, p->inv, p->nlevs, n,
+                                                            sc.variant == SPTRSV_VAR_MULTIROW, b, x, x64, s);
+        }
+    }
+    // the kernels below wait on x itself: not ready is all ones
+    SPT_CUDA(cudaMemsetAsync(x, 0xFF, sizeof(T) * (size_t)n * nrhs, s));
     if (sc.variant == SPTRSV_VAR_CLUSTER && nrhs == 1) {
         int e = build_cluster_layout(p, sc.band_levels, sc.cluster_rows);
         if (!e) e = build_cluster_tasks(p, sc.rows_per_warp);
@@ -531,7 +618,6 @@ int part_scatter32(PartPlan* q, const float* src, float* out32, double* x64, int
 int plan_solve_f64(sptrsv_plan_s* p, const double* b, double* x, int nrhs, cudaStream_t s)
 {
     if (partitioned(p)) return part_solve_f64(p, b, x, nrhs, s);
-    SPT_CUDA(cudaMemsetAsync(x, 0xFF, sizeof(double) * (size_t)p->n * nrhs, s));
     return plan_launch<double, double, double, OUT_X>(p, false, b, x, nullptr, nrhs, s);
 }
 
@@ -566,7 +652,6 @@ int part_solve32(sptrsv_plan_s* p, const BT* rhs, float* out32, double* x64, int
         g = q->bx32;
     }
     if (e) return e;
-    SPT_CUDA(cudaMemsetAsync(q->xx32, 0xFF, sizeof(float) * (size_t)q->n_ext * nrhs, s));
     e = plan_launch<float, float, BT, OUT_X>(q->sub, true, g, q->xx32, nullptr, nrhs, s);
     if (e) return e;
     return part_scatter32(q, q->xx32, out32, x64, out_mode, nrhs, s);
@@ -580,7 +665,6 @@ template <typename BT>
 int solve32(sptrsv_plan_s* p, const BT* rhs, float* out32, double* x64, int out_mode, int nrhs, cudaStream_t s)
 {
     if (partitioned(p)) return part_solve32<BT>(p, rhs, out32, x64, out_mode, nrhs, s);
-    SPT_CUDA(cudaMemsetAsync(out32, 0xFF, sizeof(float) * (size_t)p->n * nrhs, s));
     if (out_mode == OUT_SET64) return plan_launch<float, float, BT, OUT_SET64>(p, true, rhs, out32, x64, nrhs, s);
     if (out_mode == OUT_ADD64) return plan_launch<float, float, BT, OUT_ADD64>(p, true, rhs, out32, x64, nrhs, s);
     return plan_launch<float, float, BT, OUT_X>(p, true, rhs, out32, nullptr, nrhs, s);
@@ -772,6 +856,8 @@ int sptrsv_plan_create(const sp_mat_t* L, const dfr_analysis_info_t* info, sptrs
         }
         PCHK(dalloc(&p->inv, n));
         PCHK(dalloc(&p->levels, n));
+        PCHK(dalloc(&p->lptr, (long long)p->nlevs + 1));
+        std::copy(rec->stats, rec->stats + 16, p->stats);
         PCHK(dalloc(&p->ibase, (long long)p->n_warps + 1));
         PCHK(dalloc(&p->ivect, p->n_warps));
         PCHK(dalloc(&d_scr, scan_scratch_ints((long long)n + 1)));
@@ -783,6 +869,7 @@ int sptrsv_plan_create(const sp_mat_t* L, const dfr_analysis_info_t* info, sptrs
             if (e) return fail(e);
             PCHK(cudaMemcpyAsync(p->inv, info->inv_iorder, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, s));
             PCHK(cudaMemcpyAsync(p->levels, rec->d_levels, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, s));
+            PCHK(cudaMemcpyAsync(p->lptr, rec->d_lptr, sizeof(int) * ((size_t)p->nlevs + 1), cudaMemcpyDeviceToDevice, s));
         }
         PCHK(cudaMemcpyAsync(p->ibase, rec->d_ibase, sizeof(int) * ((size_t)p->n_warps + 1), cudaMemcpyDeviceToDevice, s));
         if (p->n_warps > 0)

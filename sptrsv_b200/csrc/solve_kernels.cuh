@@ -56,6 +56,15 @@ struct NatMat {
     __device__ __forceinline__ double inv(const RowRef& q) const { return 1.0 / __ldg(val + q.d); }
     __device__ __forceinline__ int c(int p) const { return __ldg(col + p); }
     __device__ __forceinline__ double v(int p) const { return __ldg(val + p); }
+    // row() in steps, for callers that load each step ahead (k_sptrsv_level_cta)
+    static constexpr bool kInvStored = false;  // scale() is the diagonal
+    __device__ __forceinline__ int id(int pos) const { return seq ? __ldg(seq + pos) : pos; }
+    __device__ __forceinline__ void range(int, int r, int& s, int& e) const
+    {
+        s = __ldg(rowptr + r);
+        e = __ldg(rowptr + r + 1) - 1;
+    }
+    __device__ __forceinline__ double scale(int, int e) const { return __ldg(val + e); }
 };
 
 template <typename VT>
@@ -82,6 +91,14 @@ struct PermMat {
     __device__ __forceinline__ VT diag(const RowRef& q) const { return __ldg(dg + q.d); }
     __device__ __forceinline__ int c(int p) const { return __ldg(col + p); }
     __device__ __forceinline__ VT v(int p) const { return __ldg(val + p); }
+    static constexpr bool kInvStored = true;  // layout order only (seq null)
+    __device__ __forceinline__ int id(int pos) const { return __ldg(rowid + pos); }
+    __device__ __forceinline__ void range(int pos, int, int& s, int& e) const
+    {
+        s = __ldg(ptr + pos);
+        e = __ldg(ptr + pos + 1);
+    }
+    __device__ __forceinline__ VT scale(int pos, int) const { return __ldg(di + pos); }
 };
 
 // Output modes: write x only; also x64 = x; also x64 += x.
