@@ -9,14 +9,14 @@
 // a status word) lives in one file-scope __device__ array of fixed size,
 // which every GPU that loads this library keeps for the life of the process.
 //
-// The solve needs no analysis and no plan: an FP32 solve over natural-order
-// chunks (the SIMPLE schedule, values read from the caller's FP64 CSR and
+// The solve needs no analysis and no plan: an FP32 solve in natural order
+// (the SIMPLE schedule, values read from the caller's FP64 CSR and
 // rounded on the fly), then ir_iters times an FP64 residual r = b - L x and
 // an FP32 correction solve with x += d in FP64.
 #include <mutex>
 
 #include "internal.h"
-#include "solve_kernels.cuh"
+#include "natural.cuh"
 
 namespace sptrsv {
 
@@ -87,30 +87,30 @@ __global__ void __launch_bounds__(256) k_residual_nat(const int* __restrict__ ro
     }
 }
 
-// Chunk solve over the natural order with an explicit grid (no occupancy
-// cache, no cooperative attribute bookkeeping beyond the launch itself).
+// Natural-order solve with an explicit grid (no occupancy cache, no
+// cooperative attribute bookkeeping beyond the launch itself).
 template <typename BT, int OUT>
-cudaError_t launch_chunk(const NatMat& m, int n, const BT* b, float* x32, double* x, DevStatus* st, int sms,
+cudaError_t launch_natural(const NatMat& m, int n, const BT* b, float* x32, double* x, DevStatus* st, int sms,
                          cudaStream_t s)
 {
-    auto kern = k_sptrsv_chunk<NatMat, float, BT, OUT, true>;
+    auto kern = k_sptrsv_natural<NatMat, float, BT, OUT, true, false>;
     int per_sm = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kNatGroup, 0);
     if (e != cudaSuccess) return e;
-    long long need = ((long long)(n + 31) / 32 + 7) / 8;
+    long long need = ((long long)n + kNatGroup - 1) / kNatGroup;
     long long grid = (long long)per_sm * sms;
     if (grid > need) grid = need;
     if (grid < 1) grid = 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(kNatGroup);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, m, n, 32, b, x32, x, st, wait_budget_ns(), 0u);
+    return cudaLaunchKernelEx(&cfg, kern, m, n, b, x32, x, st, wait_budget_ns());
 }
 
 }  // namespace
@@ -143,14 +143,14 @@ extern "C" int sptrsv_solve_ir_noalloc(const sp_mat_t* L, const double* b, doubl
         SPT_CUDA(cudaMemsetAsync(st, 0, sizeof(DevStatus), stream));
         SPT_CUDA(cudaMemsetAsync(x32, 0xFF, sizeof(float) * (size_t)n, stream));
         NatMat m{L->ia, L->ja, L->a, nullptr, L->nnz};
-        SPT_CUDA((launch_chunk<double, OUT_SET64>(m, n, b, x32, x, st, sms, stream)));
+        SPT_CUDA((launch_natural<double, OUT_SET64>(m, n, b, x32, x, st, sms, stream)));
         long long rgrid = ((long long)n * 32 + 255) / 256;  // one warp per row, at most 16 blocks per SM
         if (rgrid > 16LL * sms) rgrid = 16LL * sms;
         for (int it = 0; it < ir_iters; it++) {
             k_residual_nat<<<(int)rgrid, 256, 0, stream>>>(L->ia, L->ja, L->a, n, L->nnz, b, x, r32, st);
             SPT_CUDA(cudaGetLastError());
             SPT_CUDA(cudaMemsetAsync(x32, 0xFF, sizeof(float) * (size_t)n, stream));
-            SPT_CUDA((launch_chunk<float, OUT_ADD64>(m, n, r32, x32, x, st, sms, stream)));
+            SPT_CUDA((launch_natural<float, OUT_ADD64>(m, n, r32, x32, x, st, sms, stream)));
         }
         DevStatus h{};
         SPT_CUDA(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, stream));

@@ -6,6 +6,7 @@
 
 #include "internal.h"
 #include "level_cta.cuh"
+#include "natural.cuh"
 #include "plan.h"
 #include "solve_kernels.cuh"
 
@@ -38,6 +39,16 @@ int stream_seg_rows(const sptrsv_plan_s* p)
 size_t strip_smem_bytes(const sptrsv_schedule_t* s, size_t elem)
 {
     return (size_t)s->block_warps * 2 * s->rows_per_warp * 32 * elem;
+}
+
+// Opt-in to large dynamic shared memory.  The default limit covers static
+// plus dynamic shared memory up to 48 KB, so a kernel with static shared
+// memory needs the opt-in a little below that.
+template <typename K>
+cudaError_t allow_smem(K kern, size_t bytes)
+{
+    if (bytes <= 32 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 __global__ void k_iorder_level_keys(const int* __restrict__ iorder, const int* __restrict__ level, int n,
@@ -188,14 +199,14 @@ int solve_reference(sp_mat_t* mat, dfr_analysis_info_t* info, const double* b, d
         SPT_CUDA(launch_persistent(kern, kRefBlock, 0, div_up(n, kRefWarps), s, m, n, n, 32, (const int*)nullptr,
                                    (const int*)nullptr, b, x, (double*)nullptr, c->d_status, budget, 0u));
     } else {
-        // SIMPLE (solve_csr_simple.cu:10-108) walks the natural order in
-        // chunks: the reference gives a block a run of rows and resolves
-        // dependencies inside the block through shared memory; here a warp
-        // takes 32 consecutive rows, solves them in sequence and reads
-        // in-chunk dependencies from its shared-memory ring
-        auto kc = k_sptrsv_chunk<NatMat, double, double, OUT_X>;
-        SPT_CUDA(launch_persistent(kc, kRefBlock, 0, div_up(div_up(n, 32), kRefWarps), s, m, n, 32, b, x,
-                                   (double*)nullptr, c->d_status, budget, 0u));
+        // SIMPLE (solve_csr_simple.cu:10-108) walks the natural order: the
+        // reference gives a block a run of rows and resolves dependencies
+        // inside the block through shared memory; so do groups of 256 rows here
+        auto kn = k_sptrsv_natural<NatMat, double, double, OUT_X, false, true>;
+        const size_t smem = nat_stage_bytes<double>();
+        SPT_CUDA(allow_smem(kn, smem));
+        SPT_CUDA(launch_persistent(kn, kNatGroup, smem, div_up(n, kNatGroup), s, m, n, b, x, (double*)nullptr,
+                                   c->d_status, budget));
     }
     return ok();
 }
@@ -358,16 +369,6 @@ sptrsv_schedule_t default_schedule()
     s.cluster_rows = 4096;
     s.partitions = 0;
     return s;
-}
-
-// Opt-in to large dynamic shared memory.  The default limit covers static
-// plus dynamic shared memory up to 48 KB, so a kernel with static shared
-// memory needs the opt-in a little below that.
-template <typename K>
-cudaError_t allow_smem(K kern, size_t bytes)
-{
-    if (bytes <= 32 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 }  // namespace
@@ -562,10 +563,11 @@ int plan_launch(sptrsv_plan_s* p, bool f32, const BT* b, T* x, double* x64, int 
         return 0;
     }
     if (sc.variant == SPTRSV_VAR_SIMPLE) {
-        // natural-order chunks of rows_per_warp rows, solved in sequence by a warp
-        auto kern = k_sptrsv_chunk<PermMat<V>, T, BT, OUT>;
-        SPT_CUDA(launch_persistent_capped(kern, block, 0, div_up(div_up(n, sc.rows_per_warp), wpb), cap, s, m, n,
-                                          sc.rows_per_warp, b, x, x64, c->d_status, budget, backoff));
+        // natural order (rows_per_warp has no bearing on it)
+        auto kern = k_sptrsv_natural<PermMat<V>, T, BT, OUT, false, false>;
+        const int ncap = sc.warps_per_sm > 0 ? (sc.warps_per_sm + kNatGroup / 32 - 1) / (kNatGroup / 32) : 0;
+        SPT_CUDA(launch_persistent_capped(kern, kNatGroup, 0, div_up(n, kNatGroup), ncap, s, m, n, b, x, x64,
+                                          c->d_status, budget));
         return 0;
     }
     auto kern = k_sptrsv<PermMat<V>, T, BT, OUT>;

@@ -860,103 +860,6 @@ __global__ void __launch_bounds__(512, 1) k_sptrsv_wave(WaveMat<V> w, int ngroup
     }
 }
 
-// Natural-order chunks (the plan's SIMPLE schedule): warp task t covers the
-// natural rows [t*R, t*R+R) and solves them one after another with all 32
-// lanes striding each row's elements.  A dependency inside the chunk was
-// solved by this warp a moment ago and is read from the warp's shared-memory
-// ring without waiting; others are polled warp-convergently.  The next row's
-// metadata and first elements are loaded while the current row waits.
-//
-// CHECK (NatMat only; for callers whose CSR was never validated on the host):
-// before a row's entries are touched, its range must satisfy
-// 0 <= rowptr[r] < rowptr[r+1] <= nnz with the diagonal last
-// (col[rowptr[r+1]-1] == r), and every off-diagonal column must satisfy
-// 0 <= c < r before it indexes the ring or x.  A violation records
-// SPTRSV_ERR_INVALID_CSR and the row in the status word and the warp leaves
-// without any access through the bad index.
-template <class M, typename T, typename BT, int OUT, bool CHECK = false>
-__global__ void __launch_bounds__(512) k_sptrsv_chunk(M m, int n, int R, const BT* __restrict__ b, T* x, double* x64,
-                                                      DevStatus* st, unsigned long long budget, unsigned backoff)
-{
-    __shared__ T ring[16][32];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    T* my = ring[wib];
-    const int gw = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    const int nw = (int)(((long long)gridDim.x * blockDim.x) >> 5);
-    const int ntasks = (n + R - 1) / R;
-    for (int t = gw; t < ntasks; t += nw) {
-        const int r0 = t * R, cnt = min(R, n - r0);
-        // row j of the chunk: metadata in lane j (cnt <= 32)
-        RowRef mq;
-        mq.s = mq.e = 0;
-        T mpiv = 0, mb = 0;
-        bool bad = false;
-        if (lane < cnt) {
-            mq = m.row(r0 + lane);
-            if constexpr (CHECK) bad = !(mq.s >= 0 && mq.s <= mq.e && mq.e < m.nnz) || m.c(mq.e) != mq.r;
-            if (!bad) {
-                mpiv = (T)m.inv(mq);
-                mb = (T)b[mq.r];
-            }
-        }
-        if constexpr (CHECK) {
-            const unsigned badm = __ballot_sync(0xffffffffu, bad);
-            if (badm) {
-                if (lane == __ffs(badm) - 1) report(st, SPTRSV_ERR_INVALID_CSR, mq.r);
-                return;
-            }
-        }
-        int ns = __shfl_sync(0xffffffffu, mq.s, 0), ne = __shfl_sync(0xffffffffu, mq.e, 0);
-        int nc = 0;
-        T nv = 0;
-        if (ns + lane < ne) {
-            nc = m.c(ns + lane);
-            nv = (T)m.v(ns + lane);
-        }
-        for (int j = 0; j < cnt; j++) {
-            const int s = ns, e = ne;
-            int c = nc;
-            T v = nv;
-            const T piv = __shfl_sync(0xffffffffu, mpiv, j);
-            const T bj = __shfl_sync(0xffffffffu, mb, j);
-            T acc = lane == 0 ? bj : (T)0;
-            if (j + 1 < cnt) {  // prefetch the next row's first elements
-                ns = __shfl_sync(0xffffffffu, mq.s, j + 1);
-                ne = __shfl_sync(0xffffffffu, mq.e, j + 1);
-                if (ns + lane < ne) {
-                    nc = m.c(ns + lane);
-                    nv = (T)m.v(ns + lane);
-                }
-            }
-            for (int p = s + lane, first = 1; __any_sync(0xffffffffu, p < e); p += 32, first = 0) {
-                const bool have = p < e;
-                if (have && !first) {
-                    c = m.c(p);
-                    v = (T)m.v(p);
-                }
-                if constexpr (CHECK) {
-                    const unsigned badm = __ballot_sync(0xffffffffu, have && (c < 0 || c >= r0 + j));
-                    if (badm) {
-                        if (lane == __ffs(badm) - 1) report(st, SPTRSV_ERR_INVALID_CSR, r0 + j);
-                        return;
-                    }
-                }
-                const bool local = have && c >= r0;
-                T xv = local ? my[c - r0] : (T)0;
-                if (!warp_wait<false, T>(have && !local, c, x, nullptr, xv, st, budget, backoff, r0 + j)) return;
-                if (have) acc -= v * xv;
-            }
-            for (int o = 16; o >= 1; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-            if (lane == 0) {
-                T val = publishable(acc * piv);
-                my[j] = val;
-                publish<T, OUT>(x, x64, (size_t)(r0 + j), val);
-            }
-            __syncwarp();
-        }
-    }
-}
-
 // FP64 residual r = b - L x over a plan layout (columns must be global);
 // L lanes per row (single RHS) or one lane per right-hand side (K > 1).
 template <typename RT>

@@ -35,7 +35,7 @@ int sptrsv_schedule_from_class(int cls, sptrsv_schedule_t* s)
         if (!s || cls < 0 || cls >= SPTRSV_N_CLASSES) return set_error(SPTRSV_ERR_INVALID_ARG, "schedule_from_class: bad class");
         // preset: {variant, rows_per_warp, block_warps, warps_per_sm, backoff_ns, band_levels, cluster_rows, partitions}
         static const int T[SPTRSV_N_CLASSES][8] = {
-            // natural order / wavefront: SIMPLE 32 rows per task, STRIP one line per warp, WAVE 8 and 4 lines
+            // natural order / wavefront: SIMPLE natural-order groups, STRIP one line per warp, WAVE 8 and 4 lines
             // per CTA, and WAVE over 16 blocks with warm-ups (4 and 8 lines per CTA)
             {SPTRSV_VAR_SIMPLE, 32, 8, 0, 0, 64, 4096, 0},   {SPTRSV_VAR_STRIP, 1, 2, 0, 0, 64, 4096, 0},
             {SPTRSV_VAR_WAVE, 1, 8, 0, 0, 64, 4096, 0},      {SPTRSV_VAR_WAVE, 1, 4, 0, 0, 64, 4096, 0},
