@@ -1,40 +1,45 @@
-// band.cu — the BAND schedule: one warp per independent unit of rows, level
-// by level, x in a shared-memory ring, records streamed in by bulk copies.
+// band.cu — the BAND schedule: one CTA per independent unit of rows, its
+// steps handed from warp to warp, x in shared-memory slots.
 //
 // A unit is a set of consecutive rows that depends on no row outside it:
 // the whole matrix, or one block of a partitioned plan's block system.  One
-// warp (one CTA of 32 threads) solves its unit alone, so no flag, poll or
-// wait on another warp exists anywhere: the warp takes the unit's levels in
-// order and, between levels, only a __syncwarp orders its shared-memory
-// writes before the next level's reads.  The cost of a dependent step is a
-// shared-memory load, U fused multiply-adds, a short shuffle reduction and
-// a shared-memory store (about 100-150 cycles), against a cross-warp hop
-// through L2 of about 0.4 us in the level-ordered kernels.  It suits units
-// whose levels are narrow (banded matrices: about 16 rows per level).
+// CTA solves its unit alone, so no flag, poll or wait on another CTA exists
+// anywhere.  The unit's rows are cut into steps of at most 32/kp rows with kp
+// lanes per row (at most U = 4 entries per lane), every row after the steps of
+// the rows it reads, and step t is warp t mod 8's.  While the others work on
+// the steps before, a warp has its next two steps' records and its next
+// step's right-hand sides on their way into registers; between two steps only
+// this is left: a named barrier (about 25 cycles), shared-memory loads of x,
+// products, lane reduction, one shared-memory store, arrival at the next
+// warp's barrier.  It suits units whose levels are narrow (banded matrices:
+// about 16 rows per level).
 //
-// Records.  A unit's levels are cut into steps of at most 32/kp rows with
-// kp lanes per row (the smallest power of two that gives every row of the
-// level at most U = 4 entries per lane); step t is one fixed-size record
-// holding, per lane, a packet of 16-byte pieces stored piece-major (see
-// band_rec_bytes): the lane's 4 entry values and their columns' slots (slot
-// R holds a constant 0 for unused entries), the slot and output row of the
-// lane's row (-1: a warm-up row, x goes nowhere), 1 / L_rr, the step's kp
-// and whether it ends its level, and b of the row, written before each solve
-// by k_band_gather from bidx (the row whose b it is).  A lane reads its
-// packet with 3-4 conflict-free 128-bit loads.  The records of CH
-// consecutive steps are one contiguous chunk; lane 0 brings chunks into NST
-// shared-memory stages with cp.async.bulk (the bulk-copy engine, completion
-// counted on an mbarrier), NST - 1 chunks ahead of the warp.  The waits on
-// the mbarriers are bounded like every other wait of the library.
+// Bound: that chain, as many times as the unit has steps: 240 cycles a step,
+// against 390-480 when one warp took the steps and their records by itself
+// (unpacking a record and issuing the next one's loads stood between its
+// steps).  Steps are filled by list scheduling: of the rows that are ready,
+// those with the longest chain of readers first, whatever their level, so a
+// level of 17 rows does not cost two steps.  Banded n = 1e5 (8 in 256) over
+// 128 blocks: 153 -> 82 us, whole: 1.80 -> 0.99 ms.
 //
-// Slots.  A row's value lives in a shared-memory slot from its level until
-// the last level that reads it.  The builder hands slots out in the warp's
-// write order from a free list and takes a slot back at the first level past
-// its occupant's last reader (interval allocation over the level order), so
-// R = the most values alive at once (at most 8192); slot R holds 0 for
-// unused entries.
+// Records.  Step t is one fixed-size record holding, per lane, a packet of
+// 16-byte pieces stored piece-major (see band_rec_bytes): the lane's 4 entry
+// values and their columns' slots (slot R holds a constant 0 for unused
+// entries), the slot of the lane's row, the row of b and x it takes (-1:
+// none), whether x is written (a warm-up row's is not), 1 / L_rr and the
+// step's kp.  A lane reads its packet with 3-4 coalesced 128-bit loads.
+//
+// Slots.  A row's value lives in a shared-memory slot from its step until
+// the last step that reads it.  The builder hands slots out in step order from
+// a free list and takes a slot back after its occupant's last reader (interval
+// allocation), so R = the most values alive at once (at most 8192); slot R
+// holds 0 for unused entries.  Where list scheduling keeps more than that
+// alive, the steps follow the levels.
 #include <algorithm>
 #include <cstring>
+#include <exception>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "internal.h"
@@ -45,292 +50,312 @@ namespace sptrsv {
 
 namespace {
 
-constexpr int kBandCH = 16;       // steps per chunk
-constexpr int kBandNST = 3;       // chunk stages in shared memory
+constexpr int kBandWarps = 8;     // one hardware barrier each
 constexpr int kBandMaxRing = 8192;
 
 // Record of one step: per lane a packet of 16-byte pieces, stored piece-major
 // (piece k of lane j at k * 512 + j * 16), so a warp reads a piece with one
-// conflict-free 128-bit shared-memory load per lane.
-//   FP64 (4 pieces): {v0, v1} {v2, v3} {slot0|slot1, slot2|slot3, os|kp<<16|lend<<24, xi} {inv, bv}
-//   FP32 (3 pieces): {v0..v3} {slot0|slot1, slot2|slot3, os|kp<<16|lend<<24, xi} {inv, bv, 0, 0}
-// (slots and os 16 bits each; kp and lend are the step's, the same in every lane)
+// coalesced 128-bit load per lane.
+//   FP64 (4 pieces): {v0, v1} {v2, v3} {slot0|slot1, slot2|slot3, os|kp<<16|write<<24, row} {inv, 0}
+//   FP32 (3 pieces): {v0..v3} {slot0|slot1, slot2|slot3, os|kp<<16|write<<24, row} {inv, 0, 0, 0}
+// (slots and os 16 bits each; kp is the step's, the same in every lane)
 __host__ __device__ constexpr int band_pieces(int tsz) { return tsz == 8 ? 4 : 3; }
 __host__ __device__ constexpr int band_rec_bytes(int tsz) { return band_pieces(tsz) * 512; }
-// byte offset of lane j's b inside a record
-__host__ __device__ constexpr size_t band_bv_offset(int tsz, int j)
-{
-    return tsz == 8 ? 3 * 512 + (size_t)j * 16 + 8 : 2 * 512 + (size_t)j * 16 + 4;
-}
 
-__device__ __forceinline__ unsigned smem_addr(const void* p)
-{
-    return (unsigned)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, unsigned long long* bar)
-{
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_addr(dst)),
-        "l"(src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity)
-{
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Bounded wait for phase `parity` of an mbarrier; false when the budget ran
-// out (recorded in the status word) or another kernel reported an error.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, DevStatus* st,
-                                          unsigned long long budget, int row)
-{
-    if (mbar_try_wait(bar, parity)) return true;
-    const unsigned long long t0 = global_ns();
-    for (unsigned it = 1;; it++) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 63u) == 0) {
-            if (ld_relaxed(&st->code) != 0) return false;
-            if (global_ns() - t0 > budget) {
-                report(st, SPTRSV_ERR_TIMEOUT, row);
-                return false;
-            }
-        }
-    }
-}
-
-// b of every step's rows into the records (T = the record value type).
-template <typename T, typename BT>
-__global__ void k_band_gather(unsigned char* rec, const int* __restrict__ bidx, long long nslots,
-                              const BT* __restrict__ b)
-{
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nslots;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int r = bidx[i];
-        T* bv = reinterpret_cast<T*>(rec + (size_t)(i >> 5) * band_rec_bytes(sizeof(T)) +
-                                     band_bv_offset(sizeof(T), (int)(i & 31)));
-        *bv = r >= 0 ? (T)b[r] : (T)0;
-    }
-}
-
-// One step's record pieces of this lane, as loaded (3-4 128-bit words), and
-// unpacked into the fields the step uses (U = 4).
+// One step's record pieces of this lane.
 template <typename T>
-struct BandRaw {
-    static constexpr int NP = sizeof(T) == 8 ? 4 : 3;
+struct BandRec {
+    static constexpr int NP = sizeof(T) == 8 ? 4 : 3, META = NP - 2;
     uint4 c[NP];
     __device__ __forceinline__ void fetch(const unsigned char* r, int lane)
     {
         const uint4* p = reinterpret_cast<const uint4*>(r) + lane;
 #pragma unroll
-        for (int k = 0; k < NP; k++) c[k] = p[32 * k];
+        for (int k = 0; k < NP; k++) c[k] = __ldg(p + 32 * k);
     }
-};
-
-template <typename T>
-struct BandStep {
-    int kp, lend, os, xi;
-    T v[4], bv, inv;
-    int sl[4];
-    __device__ __forceinline__ void unpack_meta(const uint4& c)
+    __device__ __forceinline__ int row() const { return (int)c[META].w; }
+    __device__ __forceinline__ int own() const { return (int)(c[META].z & 0xffffu); }
+    __device__ __forceinline__ int kp() const { return (int)((c[META].z >> 16) & 0xffu); }
+    __device__ __forceinline__ bool write() const { return (c[META].z >> 24) != 0; }
+    __device__ __forceinline__ int slot(int q) const
     {
-        sl[0] = (int)(c.x & 0xffffu);
-        sl[1] = (int)(c.x >> 16);
-        sl[2] = (int)(c.y & 0xffffu);
-        sl[3] = (int)(c.y >> 16);
-        os = (int)(c.z & 0xffffu);
-        kp = (int)((c.z >> 16) & 0xffu);
-        lend = (int)(c.z >> 24);
-        xi = (int)c.w;
+        const unsigned w = q < 2 ? c[META].x : c[META].y;
+        return (int)((q & 1) ? w >> 16 : w & 0xffffu);
     }
-    __device__ __forceinline__ void unpack(const BandRaw<T>& r);
+    __device__ __forceinline__ T v(int q) const;
+    __device__ __forceinline__ T inv() const;
 };
 template <>
-__device__ __forceinline__ void BandStep<double>::unpack(const BandRaw<double>& r)
+__device__ __forceinline__ double BandRec<double>::v(int q) const
 {
-    v[0] = __hiloint2double((int)r.c[0].y, (int)r.c[0].x);
-    v[1] = __hiloint2double((int)r.c[0].w, (int)r.c[0].z);
-    v[2] = __hiloint2double((int)r.c[1].y, (int)r.c[1].x);
-    v[3] = __hiloint2double((int)r.c[1].w, (int)r.c[1].z);
-    unpack_meta(r.c[2]);
-    inv = __hiloint2double((int)r.c[3].y, (int)r.c[3].x);
-    bv = __hiloint2double((int)r.c[3].w, (int)r.c[3].z);
+    const uint4& p = c[q >> 1];
+    return (q & 1) ? __hiloint2double((int)p.w, (int)p.z) : __hiloint2double((int)p.y, (int)p.x);
 }
 template <>
-__device__ __forceinline__ void BandStep<float>::unpack(const BandRaw<float>& r)
+__device__ __forceinline__ double BandRec<double>::inv() const
 {
-    v[0] = __uint_as_float(r.c[0].x);
-    v[1] = __uint_as_float(r.c[0].y);
-    v[2] = __uint_as_float(r.c[0].z);
-    v[3] = __uint_as_float(r.c[0].w);
-    unpack_meta(r.c[1]);
-    inv = __uint_as_float(r.c[2].x);
-    bv = __uint_as_float(r.c[2].y);
+    return __hiloint2double((int)c[3].y, (int)c[3].x);
+}
+template <>
+__device__ __forceinline__ float BandRec<float>::v(int q) const
+{
+    return __uint_as_float(q == 0 ? c[0].x : q == 1 ? c[0].y : q == 2 ? c[0].z : c[0].w);
+}
+template <>
+__device__ __forceinline__ float BandRec<float>::inv() const
+{
+    return __uint_as_float(c[2].x);
 }
 
-template <typename T, int U, int OUT>
-__global__ void __launch_bounds__(32) k_sptrsv_band(const unsigned char* __restrict__ rec,
-                                                    const int* __restrict__ ustep, int nunits, int R, T* x,
-                                                    double* x64, DevStatus* st, unsigned long long budget)
+template <typename T, typename BT, int OUT>
+__global__ void __launch_bounds__(32 * kBandWarps) k_sptrsv_band(const unsigned char* __restrict__ rec,
+                                                                const int* __restrict__ ustep, int R,
+                                                                const BT* __restrict__ b, T* x, double* x64)
 {
     constexpr int rec_bytes = band_rec_bytes(sizeof(T));
     extern __shared__ __align__(16) unsigned char sm[];
-    __shared__ __align__(8) unsigned long long bars[kBandNST];
-    const int lane = threadIdx.x;
-    T* ring = reinterpret_cast<T*>(sm);
-    unsigned char* stage = sm + (((size_t)(R + 1) * sizeof(T) + 15) & ~(size_t)15);
-    const size_t chunk_bytes = (size_t)kBandCH * rec_bytes;
-    if (lane == 0) {
-        for (int k = 0; k < kBandNST; k++) mbar_init(&bars[k], 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    volatile T* ring = reinterpret_cast<volatile T*>(sm);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int t0 = __ldg(ustep + blockIdx.x), ns = __ldg(ustep + blockIdx.x + 1) - t0;
+    if (threadIdx.x == 0) ring[R] = (T)0;
+    __syncthreads();
+    BandRec<T> nxt, aft;  // the warp's next step and the one after
+    T bn = (T)0;          // the next step's right-hand side
+    auto rhs = [&](const BandRec<T>& z) -> T { return z.row() >= 0 ? (T)__ldg(b + z.row()) : (T)0; };
+    if (warp < ns) {
+        nxt.fetch(rec + (size_t)(t0 + warp) * rec_bytes, lane);
+        bn = rhs(nxt);
     }
-    __syncwarp();
-    unsigned long long used = 0;  // chunks this CTA has consumed (stage = used % NST, parity from used / NST)
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-        const int t0 = __ldg(ustep + u), t1 = __ldg(ustep + u + 1);
-        const int nch = (t1 - t0 + kBandCH - 1) / kBandCH;
-        if (lane == 0) ring[R] = (T)0;
-        auto issue = [&](int c) {  // lane 0: chunk c of this unit into its stage
-            const unsigned long long g = used + c;
-            const int k = (int)(g % kBandNST);
-            const int steps = min(kBandCH, t1 - t0 - c * kBandCH);
-            const unsigned bytes = (unsigned)((size_t)steps * rec_bytes);
-            mbar_expect_tx(&bars[k], bytes);
-            bulk_g2s(stage + k * chunk_bytes, rec + (size_t)(t0 + c * kBandCH) * rec_bytes, bytes, &bars[k]);
-        };
-        if (lane == 0)
-            for (int c = 0; c < min(nch, kBandNST - 1); c++) issue(c);
-        __syncwarp();
-        bool failed = false;
-        int cfail = 0;
-        for (int c = 0; c < nch; c++) {
-            // keep NST - 1 chunks in flight: the stage of chunk c + NST - 1 was
-            // last read at chunk c - 1 (the __syncwarp below ordered those reads;
-            // the proxy fence orders them before the bulk copy's writes)
-            if (lane == 0 && c + kBandNST - 1 < nch) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                issue(c + kBandNST - 1);
-            }
-            const unsigned long long g = used + c;
-            const int k = (int)(g % kBandNST);
-            const unsigned parity = (unsigned)((g / kBandNST) & 1ull);
-            int ok = 1;
-            if (lane == 0) ok = mbar_wait(&bars[k], parity, st, budget, u);
-            if (!__shfl_sync(0xffffffffu, ok, 0)) {
-                failed = true;
-                cfail = c;
-                break;
-            }
-            const unsigned char* cb = stage + k * chunk_bytes;
-            const int steps = min(kBandCH, t1 - t0 - c * kBandCH);
-            // Per step, in issue order: the next record's loads, this step's
-            // slot loads, the next record's unpacking (its loads have landed by
-            // then), the sums, the slot store.  So the chain from one level's
-            // store to the next level's slot loads holds no other instruction.
-            // A chunk's results stay in registers and go to x after its last
-            // step, outside the level-to-level chain.
-            BandStep<T> cur, nxt;
-            BandRaw<T> raw;
-            raw.fetch(cb, lane);
-            cur.unpack(raw);
-            T ov[kBandCH];
-            int oi[kBandCH];
-#pragma unroll
-            for (int j = 0; j < kBandCH; j++) {
-                oi[j] = -1;
-                if (j < steps) {
-                    if (j + 1 < steps) raw.fetch(cb + (size_t)(j + 1) * rec_bytes, lane);
-                    T rv[U];
-#pragma unroll
-                    for (int q = 0; q < U; q++) rv[q] = ring[cur.sl[q]];
-                    if (j + 1 < steps) nxt.unpack(raw);
-                    // two partial sums halve the dependent multiply-add chain
-                    T a0 = cur.bv, a1 = (T)0;
-#pragma unroll
-                    for (int q = 0; q < U; q += 2) {
-                        a0 -= cur.v[q] * rv[q];
-                        if (q + 1 < U) a1 -= cur.v[q + 1] * rv[q + 1];
-                    }
-                    T acc = a0 + a1;
-                    for (int o = cur.kp >> 1; o >= 1; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-                    if ((lane & (cur.kp - 1)) == 0 && cur.os < R) {
-                        const T xv = acc * cur.inv;
-                        ring[cur.os] = xv;
-                        ov[j] = xv;
-                        oi[j] = cur.xi;
-                    }
-                    if (cur.lend) __syncwarp();
-                    cur = nxt;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < kBandCH; j++) {
-                if (oi[j] >= 0) {
-                    if (x) x[oi[j]] = ov[j];
-                    if (OUT == OUT_SET64) x64[oi[j]] = (double)ov[j];
-                    if (OUT == OUT_ADD64) x64[oi[j]] += (double)ov[j];
-                }
-            }
-            __syncwarp();
+    if (warp + kBandWarps < ns) aft.fetch(rec + (size_t)(t0 + warp + kBandWarps) * rec_bytes, lane);
+    for (int s = warp; s < ns; s += kBandWarps) {
+        const BandRec<T> cur = nxt;
+        const T bv = bn;
+        if (s + kBandWarps < ns) {
+            nxt = aft;
+            bn = rhs(nxt);
         }
-        if (failed) {
-            // the chunks issued but not consumed, [cf, min(cf + NST, nch)), may
-            // still be landing in shared memory: wait for them (bounded, 1 s)
-            // before the CTA ends
-            if (lane == 0) {
-                const unsigned long long t_end = global_ns() + 1000000000ull;
-                for (int c = cfail; c < min(cfail + kBandNST, nch); c++) {
-                    const unsigned long long g = used + c;
-                    const unsigned par = (unsigned)((g / kBandNST) & 1ull);
-                    while (!mbar_try_wait(&bars[g % kBandNST], par) && global_ns() < t_end) {
+        if (s + 2 * kBandWarps < ns) aft.fetch(rec + (size_t)(t0 + s + 2 * kBandWarps) * rec_bytes, lane);
+        const T v0 = -cur.v(0), v1 = -cur.v(1), v2 = -cur.v(2), v3 = -cur.v(3), inv = cur.inv();
+        const int s0 = cur.slot(0), s1 = cur.slot(1), s2 = cur.slot(2), s3 = cur.slot(3);
+        const int kp = cur.kp(), own = cur.own();
+        const bool mine = own < R;
+        if (s > 0) asm volatile("barrier.cta.sync %0, 64;" ::"r"(warp) : "memory");
+        const T x0 = ring[s0], x1 = ring[s1], x2 = ring[s2], x3 = ring[s3];
+        // two partial sums halve the dependent multiply-add chain
+        T a0 = bv + v0 * x0, a1 = v1 * x1;
+        a0 += v2 * x2;
+        a1 += v3 * x3;
+        T acc = a0 + a1;
+        if (kp > 1) {
+            if (kp > 2) {
+                if (kp > 4) {
+                    if (kp > 8) {
+                        if (kp > 16) acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+                        acc += __shfl_xor_sync(0xffffffffu, acc, 8);
                     }
+                    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
                 }
+                acc += __shfl_xor_sync(0xffffffffu, acc, 2);
             }
-            __syncwarp();
-            return;
+            acc += __shfl_xor_sync(0xffffffffu, acc, 1);
         }
-        used += nch;
+        const T xv = acc * inv;
+        if (mine) ring[own] = xv;
+        if (s + 1 < ns)
+            asm volatile("barrier.cta.arrive %0, 64;" ::"r"((warp + 1) % kBandWarps) : "memory");
+        if (cur.write()) {
+            const int r = cur.row();
+            if (x) x[r] = xv;
+            if (OUT == OUT_SET64) x64[r] = (double)xv;
+            if (OUT == OUT_ADD64) x64[r] += (double)xv;
+        }
     }
 }
 
-template <typename T, int OUT>
-int band_launch_t(const BandLayout& t, const unsigned char* rec, int rb, T* x, double* x64, cudaStream_t s)
+template <typename T, typename BT, int OUT>
+int band_launch_t(const BandLayout& t, const unsigned char* rec, const BT* b, T* x, double* x64, cudaStream_t s)
 {
-    Ctx* c = ctx();
-    auto kern = k_sptrsv_band<T, kBandU, OUT>;
-    const size_t smem = (((size_t)(t.R + 1) * sizeof(T) + 15) & ~(size_t)15) + (size_t)kBandNST * kBandCH * rb;
-    SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<t.nunits, 32, smem, s>>>(rec, t.ustep, t.nunits, t.R, x, x64, c->d_status, wait_budget_ns());
+    auto kern = k_sptrsv_band<T, BT, OUT>;
+    const size_t smem = (size_t)(t.R + 1) * sizeof(T);
+    if (smem > 32 * 1024) SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<t.nunits, 32 * kBandWarps, smem, s>>>(rec, t.ustep, t.R, b, x, x64);
     SPT_CUDA(cudaGetLastError());
     return 0;
+}
+
+// One step: rows [first, first + cnt) of the unit's step order, kp lanes each.
+struct BandStepHost {
+    int kp, first, cnt;
+};
+
+// The steps of one unit: rows [a, b) of the natural CSR, all of whose columns
+// lie in it, with their levels.
+struct BandUnit {
+    std::vector<BandStepHost> steps;
+    std::vector<int> order;    // rows in step order
+    std::vector<int> slot_of;  // by row - a
+    int R = 1;
+};
+
+int band_lanes(int len)
+{
+    int kp = 1;
+    while ((len + kp - 1) / kp > kBandU) kp *= 2;
+    return kp;
+}
+
+// List scheduling: of the rows whose columns lie in earlier steps, those with
+// the longest chain of readers first; the first one's lane count is the
+// step's, rows that need more wait.
+void band_list_steps(const int* rp, const int* ci, int a, int b, BandUnit& u)
+{
+    const int n = b - a;
+    std::vector<int> height(n, 0), missing(n), cptr(n + 1, 0);
+    int top = 0;
+    for (int r = b - 1; r >= a; r--) {
+        missing[r - a] = rp[r + 1] - 1 - rp[r];
+        top = std::max(top, height[r - a]);
+        for (int q = rp[r]; q < rp[r + 1] - 1; q++) {
+            int& h = height[ci[q] - a];
+            h = std::max(h, height[r - a] + 1);
+            cptr[ci[q] - a + 1]++;
+        }
+    }
+    for (int i = 0; i < n; i++) cptr[i + 1] += cptr[i];
+    std::vector<int> reader(cptr[n]), at(cptr.begin(), cptr.end() - 1);
+    for (int r = a; r < b; r++)
+        for (int q = rp[r]; q < rp[r + 1] - 1; q++) reader[at[ci[q] - a]++] = r;
+    std::vector<std::vector<int>> ready(top + 1);  // by height
+    for (int r = b - 1; r >= a; r--)
+        if (missing[r - a] == 0) ready[height[r - a]].push_back(r);
+    u.steps.clear();
+    u.order.clear();
+    u.order.reserve(n);
+    std::vector<int> wait;
+    int hi = top;
+    while ((int)u.order.size() < n) {
+        while (ready[hi].empty()) hi--;
+        const int first = (int)u.order.size();
+        int kp = 0, per = 0;
+        for (int h = hi; h >= 0; h--) {
+            wait.clear();
+            while (!ready[h].empty() && (kp == 0 || (int)u.order.size() - first < per)) {
+                const int r = ready[h].back();
+                ready[h].pop_back();
+                const int need = band_lanes(rp[r + 1] - 1 - rp[r]);
+                if (kp == 0) {
+                    kp = need;
+                    per = 32 / kp;
+                }
+                if (need > kp) wait.push_back(r);
+                else u.order.push_back(r);
+            }
+            for (size_t k = wait.size(); k-- > 0;) ready[h].push_back(wait[k]);
+            if ((int)u.order.size() - first >= per) break;
+        }
+        const int cnt = (int)u.order.size() - first;
+        u.steps.push_back({kp, first, cnt});
+        for (int k = first; k < first + cnt; k++) {
+            const int i = u.order[k] - a;
+            for (int q = cptr[i]; q < cptr[i + 1]; q++) {
+                const int r = reader[q];
+                if (--missing[r - a] == 0) {
+                    ready[height[r - a]].push_back(r);
+                    hi = std::max(hi, height[r - a]);
+                }
+            }
+        }
+    }
+}
+
+// Steps along the levels: every level cut by itself, its lane count from its
+// longest row.
+void band_level_steps(const int* rp, const int* lev, int a, int b, BandUnit& u)
+{
+    u.steps.clear();
+    u.order.resize(b - a);
+    for (int r = a; r < b; r++) u.order[r - a] = r;
+    std::stable_sort(u.order.begin(), u.order.end(), [&](int p, int q) { return lev[p] < lev[q]; });
+    for (int f = 0; f < b - a;) {
+        int e = f, mx = 0;
+        for (; e < b - a && lev[u.order[e]] == lev[u.order[f]]; e++)
+            mx = std::max(mx, rp[u.order[e] + 1] - 1 - rp[u.order[e]]);
+        const int kp = band_lanes(mx), per = 32 / kp;
+        for (int q = f; q < e; q += per) u.steps.push_back({kp, q, std::min(per, e - q)});
+        f = e;
+    }
+}
+
+// f(0 .. n-1) over the host's threads; what a thread throws is thrown here,
+// once all of them have ended.
+template <class F>
+void band_spread(int n, F&& f)
+{
+    const int nt = std::max(1, std::min<int>(n, (int)std::thread::hardware_concurrency()));
+    std::vector<std::exception_ptr> err(nt);
+    auto work = [&](int t) {
+        try {
+            for (int i = t; i < n; i += nt) f(i);
+        } catch (...) {
+            err[t] = std::current_exception();
+        }
+    };
+    std::vector<std::thread> th;
+    th.reserve(nt);
+    int started = 1;  // threads 1 .. started - 1 run; their shares past those are done here
+    try {
+        for (; started < nt; started++) th.emplace_back(work, started);
+    } catch (const std::system_error&) {
+    }
+    work(0);
+    for (int t = started; t < nt; t++) work(t);
+    for (auto& x : th) x.join();
+    for (auto& e : err)
+        if (e) std::rethrow_exception(e);
+}
+
+// Slots by interval allocation over the steps; false when more than
+// kBandMaxRing values are alive at once.
+bool band_slots(const int* rp, const int* ci, int a, int b, BandUnit& u)
+{
+    const int n = b - a, ns = (int)u.steps.size();
+    std::vector<int> last(n, -1), step(n);
+    for (int t = 0; t < ns; t++)
+        for (int k = u.steps[t].first; k < u.steps[t].first + u.steps[t].cnt; k++) {
+            const int r = u.order[k];
+            step[r - a] = t;
+            for (int q = rp[r]; q < rp[r + 1] - 1; q++) last[ci[q] - a] = t;  // steps ascend
+        }
+    std::vector<int> rptr(ns + 1, 0);
+    for (int i = 0; i < n; i++) rptr[std::max(last[i], step[i]) + 1]++;
+    for (int t = 0; t < ns; t++) rptr[t + 1] += rptr[t];
+    std::vector<int> rel(n), at(rptr.begin(), rptr.end() - 1), freel;
+    u.slot_of.assign(n, 0);
+    int top = 0;
+    for (int t = 0; t < ns; t++) {
+        for (int k = u.steps[t].first; k < u.steps[t].first + u.steps[t].cnt; k++) {
+            const int i = u.order[k] - a;
+            int sl;
+            if (!freel.empty()) {
+                sl = freel.back();
+                freel.pop_back();
+            } else {
+                sl = top++;
+            }
+            u.slot_of[i] = sl;
+            rel[at[std::max(last[i], t)]++] = sl;
+        }
+        for (int k = rptr[t]; k < rptr[t + 1]; k++) freel.push_back(rel[k]);  // free from the next step on
+    }
+    u.R = std::max(1, top);
+    return u.R <= kBandMaxRing;
 }
 
 }  // namespace
 
 void band_free(BandLayout& t)
 {
-    cudaFree(t.rec64); cudaFree(t.rec32); cudaFree(t.bidx); cudaFree(t.ustep);
+    cudaFree(t.rec64); cudaFree(t.rec32); cudaFree(t.ustep);
     t = BandLayout{};
 }
 
@@ -367,16 +392,6 @@ int build_band_layout(sptrsv_plan_s* p)
     if (maxoff > 32 * U)
         return set_error(SPTRSV_ERR_UNSUPPORTED, "band schedule: a row holds %d off-diagonals, more than %d", maxoff,
                          32 * U);
-    // last reader level of every row (0: never read)
-    std::vector<int> lastread(n, 0);
-    for (int r = 0; r < n; r++)
-        for (int q = rp[r]; q < rp[r + 1] - 1; q++) lastread[ci[q]] = std::max(lastread[ci[q]], lev[r]);
-    // rows of each unit by (level, row): the order the warp writes them
-    std::vector<int> all_order(n);
-    std::vector<int> ustep(nunits + 1, 0);
-    std::vector<int> lbase(nunits), lcount(nunits);  // per unit: first level, levels
-    std::vector<int> lcnt;                            // per unit and level: rows (prefix sums)
-    std::vector<size_t> lcnt_off(nunits + 1, 0);
     for (int un = 0; un < nunits; un++) {
         const int a = u0[un], b = u0[un + 1];
         int lmin = 1 << 30, lmax = 0;
@@ -387,139 +402,83 @@ int build_band_layout(sptrsv_plan_s* p)
         const int nl = b > a ? lmax - lmin + 1 : 0;
         if (b > a && (b - a) > 128 * nl)
             return set_error(SPTRSV_ERR_UNSUPPORTED, "band schedule: levels hold %d rows on average, too wide for one "
-                             "warp", (b - a) / nl);
-        lbase[un] = lmin;
-        lcount[un] = nl;
-        lcnt_off[un + 1] = lcnt_off[un] + nl + 1;
-        lcnt.resize(lcnt_off[un + 1], 0);
-        int* cnt = &lcnt[lcnt_off[un]];
-        for (int r = a; r < b; r++) cnt[lev[r] - lmin + 1]++;
-        for (int l = 0; l < nl; l++) cnt[l + 1] += cnt[l];
-        std::vector<int> pos(cnt, cnt + nl);
-        for (int r = a; r < b; r++) all_order[a + pos[lev[r] - lmin]++] = r;
+                             "CTA", (b - a) / nl);
     }
-    // shared-memory slots: a row's value lives from its write (its level)
-    // to the last level that reads it.  Slots are handed out in the warp's
-    // write order (all_order) from a free list; a slot returns to the list at
-    // the first level past its occupant's last reader, so no value is lost
-    // and R = the most values alive at once (a row nobody reads takes a slot
-    // for its own level only)
-    std::vector<int> slot_of(n, 0);
+    // the units' steps and slots, the units spread over the host's threads
+    std::vector<BandUnit> units(nunits);
+    auto spread = [&](auto&& f) { band_spread(nunits, f); };
+    spread([&](int un) {
+        const int a = u0[un], b = u0[un + 1];
+        band_list_steps(rp.data(), ci.data(), a, b, units[un]);
+        if (!band_slots(rp.data(), ci.data(), a, b, units[un])) {
+            band_level_steps(rp.data(), lev.data(), a, b, units[un]);
+            band_slots(rp.data(), ci.data(), a, b, units[un]);
+        }
+    });
     int R = 1;
-    {
-        std::vector<int> freel;
-        std::vector<std::vector<int>> release;  // per local level: slots free from the next level on
-        for (int un = 0; un < nunits; un++) {
-            const int a = u0[un], b = u0[un + 1];
-            const int nl = lcount[un], lmin = lbase[un];
-            freel.clear();
-            release.assign(nl + 1, {});
-            int top = 0, cur = -1;
-            for (int q = a; q < b; q++) {
-                const int r = all_order[q], L = lev[r] - lmin;
-                while (cur < L) {  // entering a new level: recycle slots whose readers are done
-                    if (cur >= 0)
-                        for (int x : release[cur]) freel.push_back(x);
-                    cur++;
-                }
-                int sl;
-                if (!freel.empty()) {
-                    sl = freel.back();
-                    freel.pop_back();
-                } else {
-                    sl = top++;
-                }
-                slot_of[r] = sl;
-                const int last = lastread[r] > 0 ? lastread[r] - lmin : L;  // level of its last reader
-                release[last].push_back(sl);
-            }
-            R = std::max(R, top);
-        }
-        if (R > kBandMaxRing)
-            return set_error(SPTRSV_ERR_UNSUPPORTED, "band schedule: %d values are alive at once, more than the %d "
-                             "shared-memory slots", R, kBandMaxRing);
-    }
-    struct Step {
-        int kp, level_end, first, cnt;  // rows all_order[first .. first + cnt)
-    };
-    std::vector<Step> steps;
+    std::vector<int> ustep(nunits + 1, 0);
     for (int un = 0; un < nunits; un++) {
-        const int a = u0[un];
-        const int* cnt = &lcnt[lcnt_off[un]];
-        ustep[un] = (int)steps.size();
-        for (int l = 0; l < lcount[un]; l++) {
-            const int f = a + cnt[l], L = cnt[l + 1] - cnt[l];
-            if (L == 0) continue;
-            int mx = 0;
-            for (int q = f; q < f + L; q++) {
-                const int r = all_order[q];
-                mx = std::max(mx, rp[r + 1] - rp[r] - 1);
-            }
-            int kp = 1;
-            while ((mx + kp - 1) / kp > U) kp *= 2;
-            const int per = 32 / kp;
-            for (int q = 0; q < L; q += per) steps.push_back({kp, q + per >= L ? 1 : 0, f + q, std::min(per, L - q)});
-        }
+        R = std::max(R, units[un].R);
+        ustep[un + 1] = ustep[un] + (int)units[un].steps.size();
     }
-    ustep[nunits] = (int)steps.size();
-    // the unit of each row (for the ring slot base)
-    std::vector<int> unit_of(n);
-    for (int un = 0; un < nunits; un++)
-        for (int r = u0[un]; r < u0[un + 1]; r++) unit_of[r] = un;
-    const long long ns = (long long)steps.size();
+    if (R > kBandMaxRing)
+        return set_error(SPTRSV_ERR_UNSUPPORTED, "band schedule: %d values are alive at once, more than the %d "
+                         "shared-memory slots", R, kBandMaxRing);
+    const long long ns = ustep[nunits];
     const int rb64 = band_rec_bytes(8), rb32 = band_rec_bytes(4);
     std::vector<unsigned char> h64((size_t)ns * rb64, 0), h32((size_t)ns * rb32, 0);
-    std::vector<int> bidx((size_t)ns * 32, -1);
-    for (long long t = 0; t < ns; t++) {
-        const Step& sp = steps[t];
-        unsigned char* r64 = &h64[(size_t)t * rb64];
-        unsigned char* r32 = &h32[(size_t)t * rb32];
-        // per lane: values, slots (R: the constant-0 slot), row slot, output row, 1/L_rr
-        double v[32][4] = {};
-        int sl[32][4], os[32], xi[32];
-        double inv[32] = {};
-        float invf[32] = {};
-        for (int j = 0; j < 32; j++) {
-            for (int q = 0; q < 4; q++) sl[j][q] = R;
-            os[j] = R;  // no row: slot R is never written
-            xi[j] = -1;
-        }
-        for (int w = 0; w < sp.cnt; w++) {
-            const int r = all_order[sp.first + w];
-            const int un = unit_of[r];
-            const int lane0 = w * sp.kp;
-            const int d = rp[r + 1] - 1;
-            for (int q = rp[r]; q < d; q++) {
-                const int k = q - rp[r];
-                const int lane = lane0 + (k % sp.kp), uu = k / sp.kp;
-                sl[lane][uu] = slot_of[ci[q]];
-                v[lane][uu] = va[q];
+    spread([&](int un) {
+        const BandUnit& u = units[un];
+        const int a = u0[un];
+        for (size_t t = 0; t < u.steps.size(); t++) {
+            const BandStepHost& sp = u.steps[t];
+            unsigned char* r64 = &h64[(ustep[un] + t) * rb64];
+            unsigned char* r32 = &h32[(ustep[un] + t) * rb32];
+            // per lane: values, slots (R: the constant-0 slot), row slot, outer row, 1/L_rr
+            double v[32][4] = {};
+            int sl[32][4], os[32], row[32], wr[32] = {};
+            double inv[32] = {};
+            float invf[32] = {};
+            for (int j = 0; j < 32; j++) {
+                for (int q = 0; q < 4; q++) sl[j][q] = R;
+                os[j] = R;  // no row: slot R is never written
+                row[j] = -1;
             }
-            bool real = true;
-            const int orow = outer_row(un, r, &real);
-            os[lane0] = slot_of[r];
-            xi[lane0] = real ? orow : -1;
-            inv[lane0] = 1.0 / va[d];
-            invf[lane0] = 1.0f / (float)va[d];
-            bidx[(size_t)t * 32 + lane0] = orow;
+            for (int w = 0; w < sp.cnt; w++) {
+                const int r = u.order[sp.first + w];
+                const int lane0 = w * sp.kp;
+                const int d = rp[r + 1] - 1;
+                for (int q = rp[r]; q < d; q++) {
+                    const int k = q - rp[r];
+                    const int lane = lane0 + (k % sp.kp), uu = k / sp.kp;
+                    sl[lane][uu] = u.slot_of[ci[q] - a];
+                    v[lane][uu] = va[q];
+                }
+                bool real = true;
+                row[lane0] = outer_row(un, r, &real);
+                wr[lane0] = real ? 1 : 0;
+                os[lane0] = u.slot_of[r - a];
+                inv[lane0] = 1.0 / va[d];
+                invf[lane0] = 1.0f / (float)va[d];
+            }
+            for (int j = 0; j < 32; j++) {
+                const unsigned meta[4] = {(unsigned)sl[j][0] | ((unsigned)sl[j][1] << 16),
+                                          (unsigned)sl[j][2] | ((unsigned)sl[j][3] << 16),
+                                          (unsigned)os[j] | ((unsigned)sp.kp << 16) | ((unsigned)wr[j] << 24),
+                                          (unsigned)row[j]};
+                // FP64 pieces
+                memcpy(r64 + 0 * 512 + j * 16, &v[j][0], 16);
+                memcpy(r64 + 1 * 512 + j * 16, &v[j][2], 16);
+                memcpy(r64 + 2 * 512 + j * 16, meta, 16);
+                memcpy(r64 + 3 * 512 + j * 16, &inv[j], 8);
+                // FP32 pieces
+                const float vf[4] = {(float)v[j][0], (float)v[j][1], (float)v[j][2], (float)v[j][3]};
+                memcpy(r32 + 0 * 512 + j * 16, vf, 16);
+                memcpy(r32 + 1 * 512 + j * 16, meta, 16);
+                memcpy(r32 + 2 * 512 + j * 16, &invf[j], 4);
+            }
         }
-        for (int j = 0; j < 32; j++) {
-            const unsigned meta[4] = {(unsigned)sl[j][0] | ((unsigned)sl[j][1] << 16),
-                                      (unsigned)sl[j][2] | ((unsigned)sl[j][3] << 16),
-                                      (unsigned)os[j] | ((unsigned)sp.kp << 16) | ((unsigned)sp.level_end << 24),
-                                      (unsigned)xi[j]};
-            // FP64 pieces
-            memcpy(r64 + 0 * 512 + j * 16, &v[j][0], 16);
-            memcpy(r64 + 1 * 512 + j * 16, &v[j][2], 16);
-            memcpy(r64 + 2 * 512 + j * 16, meta, 16);
-            memcpy(r64 + 3 * 512 + j * 16, &inv[j], 8);
-            // FP32 pieces
-            const float vf[4] = {(float)v[j][0], (float)v[j][1], (float)v[j][2], (float)v[j][3]};
-            memcpy(r32 + 0 * 512 + j * 16, vf, 16);
-            memcpy(r32 + 1 * 512 + j * 16, meta, 16);
-            memcpy(r32 + 2 * 512 + j * 16, &invf[j], 4);
-        }
-    }
+    });
     BandLayout t;
     t.U = U;
     t.R = R;
@@ -532,19 +491,17 @@ int build_band_layout(sptrsv_plan_s* p)
         return code;
     };
     if (dalloc(&t.ustep, nunits + 1) != cudaSuccess || dalloc(&t.rec64, (long long)ns * rb64) != cudaSuccess ||
-        dalloc(&t.rec32, (long long)ns * rb32) != cudaSuccess || dalloc(&t.bidx, ns * 32) != cudaSuccess)
+        dalloc(&t.rec32, (long long)ns * rb32) != cudaSuccess)
         return fail(cuda_fail(cudaGetLastError(), "band layout"));
     if (cudaMemcpy(t.ustep, ustep.data(), sizeof(int) * (size_t)(nunits + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
         (ns > 0 && (cudaMemcpy(t.rec64, h64.data(), h64.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-                    cudaMemcpy(t.rec32, h32.data(), h32.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-                    cudaMemcpy(t.bidx, bidx.data(), sizeof(int) * bidx.size(), cudaMemcpyHostToDevice) != cudaSuccess)))
+                    cudaMemcpy(t.rec32, h32.data(), h32.size(), cudaMemcpyHostToDevice) != cudaSuccess)))
         return fail(cuda_fail(cudaGetLastError(), "band layout upload"));
     p->band = t;
     return 0;
 }
 
-// One BAND solve: b (FP64 or FP32, indexed by the records' bidx) gathered
-// into the records of the solve's precision, then one warp per unit.
+// One BAND solve: b (FP64 or FP32, in the outer plan's rows), one CTA per unit.
 // x (T) and x64 per out_mode; x may be null.
 int band_solve(sptrsv_plan_s* p, bool f32, const void* b, bool b_f32, void* x, double* x64, int out_mode,
                cudaStream_t s)
@@ -553,22 +510,30 @@ int band_solve(sptrsv_plan_s* p, bool f32, const void* b, bool b_f32, void* x, d
     if (e) return e;
     const BandLayout& t = p->band;
     if (t.nsteps == 0) return 0;
-    const long long nslots = (long long)t.nsteps * 32;
-    const int g = grid_for(nslots, 256);
+    const double* bd = static_cast<const double*>(b);
+    const float* bf = static_cast<const float*>(b);
     if (!f32) {
-        k_band_gather<double, double><<<g, 256, 0, s>>>(t.rec64, t.bidx, nslots, static_cast<const double*>(b));
-        SPT_CUDA(cudaGetLastError());
-        return band_launch_t<double, OUT_X>(t, t.rec64, t.rb64, static_cast<double*>(x), nullptr, s);
+        double* xd = static_cast<double*>(x);
+        if (!p->part_tab.empty()) {
+            // warm-up rows read b of rows that another unit writes x of: a solve in place takes a copy of b
+            const long long m = p->part_tab[p->part_tab.size() - 2];  // end of the last block
+            if (xd < bd + m && bd < xd + m) {
+                if (!p->band_b) SPT_CUDA(dalloc(&p->band_b, m));
+                SPT_CUDA(cudaMemcpyAsync(p->band_b, bd, sizeof(double) * (size_t)m, cudaMemcpyDeviceToDevice, s));
+                bd = p->band_b;
+            }
+        }
+        return band_launch_t<double, double, OUT_X>(t, t.rec64, bd, xd, nullptr, s);
     }
-    if (b_f32)
-        k_band_gather<float, float><<<g, 256, 0, s>>>(t.rec32, t.bidx, nslots, static_cast<const float*>(b));
-    else
-        k_band_gather<float, double><<<g, 256, 0, s>>>(t.rec32, t.bidx, nslots, static_cast<const double*>(b));
-    SPT_CUDA(cudaGetLastError());
     float* xf = static_cast<float*>(x);
-    if (out_mode == OUT_SET64) return band_launch_t<float, OUT_SET64>(t, t.rec32, t.rb32, xf, x64, s);
-    if (out_mode == OUT_ADD64) return band_launch_t<float, OUT_ADD64>(t, t.rec32, t.rb32, xf, x64, s);
-    return band_launch_t<float, OUT_X>(t, t.rec32, t.rb32, xf, x64, s);
+    if (out_mode == OUT_SET64)
+        return b_f32 ? band_launch_t<float, float, OUT_SET64>(t, t.rec32, bf, xf, x64, s)
+                     : band_launch_t<float, double, OUT_SET64>(t, t.rec32, bd, xf, x64, s);
+    if (out_mode == OUT_ADD64)
+        return b_f32 ? band_launch_t<float, float, OUT_ADD64>(t, t.rec32, bf, xf, x64, s)
+                     : band_launch_t<float, double, OUT_ADD64>(t, t.rec32, bd, xf, x64, s);
+    return b_f32 ? band_launch_t<float, float, OUT_X>(t, t.rec32, bf, xf, x64, s)
+                 : band_launch_t<float, double, OUT_X>(t, t.rec32, bd, xf, x64, s);
 }
 
 }  // namespace sptrsv

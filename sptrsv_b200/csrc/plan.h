@@ -91,8 +91,8 @@ struct MrhsTable {
 };
 
 // BAND schedule (built on demand, see band.cu): per unit (the whole matrix,
-// or each block of a block system) the steps of its levels as fixed-size
-// records, FP64 and FP32 copies.
+// or each block of a block system) its steps as fixed-size records, FP64 and
+// FP32 copies.
 constexpr int kBandU = 4;  // entries per lane per step
 struct BandLayout {
     int U = 0, R = 0;          // entries per lane per step; ring slots (slot R is a constant 0)
@@ -101,7 +101,6 @@ struct BandLayout {
     unsigned char* rec64 = nullptr;  // [nsteps * rb64]
     unsigned char* rec32 = nullptr;  // [nsteps * rb32]
     int rb64 = 0, rb32 = 0;
-    int* bidx = nullptr;       // [nsteps * 32] row whose b a lane's row takes (-1: none)
 };
 
 // Partitioned solve (built on demand, see part.cu): the rows are cut into P
@@ -182,6 +181,7 @@ struct sptrsv_plan_s {
     // plan's rows directly
     std::vector<int> part_tab;
     BandLayout band;             // BAND layout (built on demand)
+    double* band_b = nullptr;    // block systems only: b of a solve in place (built on demand)
 };
 
 namespace sptrsv {

@@ -272,6 +272,7 @@ void plan_free_arrays(sptrsv_plan_s* p)
     cudaFree(p->bflag);
     part_free(p);
     band_free(p->band);
+    cudaFree(p->band_b);
     if (p->epochs) cudaFreeHost(p->epochs);
     if (p->ev_start) cudaEventDestroy(p->ev_start);
     if (p->ev_copied) cudaEventDestroy(p->ev_copied);
