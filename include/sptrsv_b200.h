@@ -348,20 +348,17 @@ int sptrsv_batch_info(sptrsv_batch_t batch, long long* offsets, int* n_total, in
 /* mode 0: level-ordered tasks over the union;
  * mode 1: each warp takes 32 consecutive rows of one system and solves them
  *         in sequence, waiting once per chunk for the chunks it reads;
- * mode 2 (default): hybrid - every system with n_s / nlevs_s below the sequential
- *         width (sptrsv_batch_set_seq_width) is solved by one warp in
- *         natural order without waiting, the others by level-ordered tasks,
- *         all in the same launch.
+ * mode 2 (default): hybrid - every system with n_s / nlevs_s below the
+ *         sequential width (sptrsv_batch_set_seq_width) is solved in natural
+ *         order by a team of warps of one block without waiting on others,
+ *         the others by level-ordered tasks, all in the same launch.
  * block_warps 2..16 (2..8 in mode 1).  Rebuilds the level layout when the
  * set of sequential systems changes. */
 int sptrsv_batch_set_schedule(sptrsv_batch_t batch, int mode, int block_warps, int warps_per_sm,
                               int backoff_ns, int ir_iters);
 /* Width threshold of mode 2 (default 16): a system is sequential when
- * n_s / nlevs_s < width and all its dependencies reach back at most
- * 1024 / kp rows (kp = power of two >= its right-hand-side count), or 1024
- * rows for a system with more than 8 right-hand sides or of at least 16384
- * rows with several (solved one right-hand side per warp); 0 makes no system
- * sequential, >= 1e9 makes every system sequential. */
+ * n_s / nlevs_s < width and all its dependencies reach back at most 1024
+ * rows; 0 makes no system sequential, >= 1e9 makes every system sequential. */
 int sptrsv_batch_set_seq_width(sptrsv_batch_t batch, double width);
 /* Systems solved sequentially, warps they occupy, rows left to the level tasks. */
 int sptrsv_batch_seq_systems(sptrsv_batch_t batch, int* nseq, int* nseq_warps, int* n_level_rows);

@@ -14,11 +14,10 @@
 // A system whose levels hold few rows on average (n_s / nlevs_s below a
 // threshold; a near-chain) gains nothing from the level order: every level
 // costs a cross-warp hop through L2.  The hybrid schedule gives each such
-// system to one warp of the same persistent launch, which walks it in natural
-// order without any wait: the values of the most recent rows stay in a
-// shared-memory ring, older ones are re-read from x (written by the same
-// warp), and row metadata is loaded a chunk of 32 rows ahead.  The other
-// systems keep the level-ordered tasks on the remaining warps.
+// system to a team of up to four warps of the same persistent launch, which
+// walks it in natural order, the rows handed on from warp to warp by named
+// barriers and the recent x values in a shared-memory ring (seq_unit).  The
+// other systems keep the level-ordered tasks on the remaining warps.
 //
 // Vectors are packed: system s owns the row-major n_s x k_s block starting at
 // element off_s (off_0 = 0, off_{s+1} = off_s + n_s k_s).  Each stored
@@ -52,7 +51,7 @@ struct sptrsv_batch_s {
     int* ptr = nullptr;
     long long* xrow = nullptr;
     int* krow = nullptr;
-    long long* xdep = nullptr;
+    void* xdep = nullptr;        // unsigned, or long long where nvec needs it
     double* val64 = nullptr;
     float* val32 = nullptr;
     double* dg64 = nullptr;
@@ -90,12 +89,14 @@ struct sptrsv_batch_s {
     std::vector<int> row0h;      // [nsys+1] first union row of each system
     std::vector<int> sys_nlev;   // [nsys] levels of each system
     std::vector<int> sys_dist;   // [nsys] largest row - column distance of an entry
-    std::vector<char> seq;       // [nsys] 1: solved by one warp in natural order (mode 2)
+    std::vector<char> seq;       // [nsys] 1: solved by a team of warps in natural order (mode 2)
     int n_lvl = 0;               // rows in the level layout (the non-sequential systems)
-    int* wptr = nullptr;         // [nseqw+1] per sequential warp: range in wsys
-    int* wsys = nullptr;         // units in sequential-warp order: system
-    int* wcol = nullptr;         // and right-hand side (-1: all of them)
-    int nseqw = 0;
+    unsigned char* late = nullptr;  // [n] entries that a team of late_w warps takes late (k_late)
+    int late_w = 0;
+    int* tptr = nullptr;         // [nteams+1] per team: range in units
+    int* units = nullptr;        // SeqUnit each: columns of a sequential system
+    int nteams = 0;
+    bool sweep = false;          // the teams are single warps (sweep_unit)
     double seq_width = 16.0;     // mode 2: sequential when n_s / nlevs_s < seq_width
     int mode = 2;                // 0: level-ordered tasks, 1: natural-order chunks, 2: hybrid
     int block_warps = 8, warps_per_sm = 0, backoff_ns = 0, ir_iters = 2;
@@ -124,32 +125,331 @@ namespace sptrsv {
 
 namespace {
 
+template <typename XI>
 struct BatchMat {
     const int* __restrict__ ptr;
     const long long* __restrict__ xrow;
     const int* __restrict__ krow;
-    const long long* __restrict__ xdep;
+    const XI* __restrict__ xdep;
 };
 
-// Systems solved by one warp each (hybrid schedule), over the natural-order
-// union without diagonals.
+// A unit of the hybrid schedule: columns [c0, c0 + kc) of a sequential system,
+// solved by one team of warps.
+struct SeqUnit {
+    int sys, c0, kc;
+    int rwlog;  // log2 of the ring's rows; + 256: some column lies further back than the ring
+};
+static_assert(sizeof(SeqUnit) == 16, "stored as four ints");
+
+// Sequential systems, over the natural-order union without diagonals.
 struct SeqSet {
     const int* __restrict__ ptr;     // nptr
     const int* __restrict__ col;     // ncol
     const int* __restrict__ row0;    // [nsys+1]
     const int* __restrict__ sk;      // [nsys]
     const long long* __restrict__ soff;
-    const int* __restrict__ wptr;    // [nseqw+1]
-    const int* __restrict__ wsys;    // per unit: system
-    const int* __restrict__ wcol;    // per unit: right-hand side (-1: all of them)
-    int nseqw;
+    const unsigned char* __restrict__ late;  // [n] entries taken late (k_late)
+    const int* __restrict__ tptr;    // [nteams+1] units of each team
+    const SeqUnit* __restrict__ units;
+    int nteams;
 };
 
-constexpr int kVkU = 8;         // elements per wait round in the level-ordered kernel
-constexpr int kSeqRing = 1024;  // ring elements per sequential warp
-constexpr int kSeqEC = 512;     // entries of one 32-row chunk that fit a stage buffer
-constexpr int kSeqMaxK = 8;     // most right-hand sides one sequential warp carries (more: one warp per column)
+constexpr int kVkU = 8;            // entries per wait round in the level-ordered kernel
+constexpr int kVkAhead = 16;       // entries of a row loaded ahead there
+constexpr int kSeqElems = 8192;    // ring elements of a team
+constexpr int kSeqMaxDist = 1024;  // furthest dependency (rows) of a system that its width makes sequential
 
+// Loads that stay where they are written: a plain load may sink to the first
+// use of its value, past the rows that are to hide it.
+__device__ __forceinline__ int load_now(const int* p)
+{
+    int v;
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int load_now(const unsigned char* p)
+{
+    unsigned short v;
+    asm volatile("ld.global.nc.u8 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float load_now(const float* p)
+{
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double load_now(const double* p)
+{
+    double v;
+    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
+
+template <typename T>
+__device__ __forceinline__ void seq_copy(T* smem, const T* g)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(g), "n"(sizeof(T)) : "memory");
+}
+
+// One entry staged in shared memory: minus its value, and its ring element
+// (~row of the system where the ring no longer holds it).
+template <typename T>
+struct alignas(2 * sizeof(T)) SeqEntry {
+    T v;
+    int at;
+};
+
+// Shared memory of a team of W warps: the ring and its zero row, then two
+// chunks of 8 W rows: entries (16 a row), 1 / diag, late counts, and three of
+// row pointers.
+template <typename T>
+struct SeqSmem {
+    static constexpr size_t al(size_t x) { return (x + 15) & ~size_t(15); }
+    static constexpr size_t ent = al((size_t)(kSeqElems + 32) * sizeof(T));
+    // per warp, four rows of right-hand sides and of the solution a correction adds to
+    static constexpr size_t rhs = 4 * 32 * 2 * sizeof(double);
+    static size_t total(int W)
+    {
+        return ent + W * rhs + 2 * 128 * W * sizeof(SeqEntry<T>) + (2 * 8 + 32) * W * sizeof(T) +
+               (2 * 8 * W + 3 * (8 * W + 1)) * sizeof(int);
+    }
+};
+
+// A team of W warps (1, 2 or 7) solves one unit in natural order, row r by
+// warp (r - first row) mod W, lane q owning column c0 + q.  The last x values
+// live in the team's shared-memory ring of rw rows (slot = row mod rw, rw at
+// least W more than the system's reach).  A row is summed in up to three
+// parts: its columns at least W rows back, whose rows this warp has seen
+// finished; with 7 warps, those 4 to 6 rows back, once row r - 4 has handed
+// over to it; and the last ones in its turn, once row r - 1 has.  A row
+// without last ones is finished before its turn and only hands on.  So between
+// two rows only this is left: a named barrier (about 60 cycles from arrival to
+// the next warp's first instruction) and, where there are last ones, their
+// products, one multiplication and one shared-memory store, whatever the
+// number of columns.  Chunks of 8 W rows (entries as {value, ring element},
+// 1 / diag, counts) are staged in shared memory a chunk ahead by the whole
+// team, row pointers two, right-hand sides three rows ahead by cp.async.  Up to
+// 16 entries a row; a chunk of more than 128 W is read from global memory.
+//
+// Bound: a warp's own instructions (about one in eight cycles): 1,550 cycles a
+// row, 222 from row to row with seven warps; the hand-over alone would allow
+// 60 to 140.  What did not do: four or eight warps that stage their own rows
+// (690 and 435 cycles a row), right-hand sides rotated through registers (the
+// loop's copies wait for the youngest load: 330).  198,324 rows of band 38, 13
+// columns: 31.0 ms as one sweeping warp a column, 22.5 ms so.
+template <typename V, typename T, typename BT, int OUT>
+__device__ __forceinline__ void seq_unit(const SeqSet& q, const V* __restrict__ val, const V* __restrict__ di,
+                                         const SeqUnit un, int W, int tw, const BT* __restrict__ b, T* x, double* x64,
+                                         unsigned char* region)
+{
+    const int lane = threadIdx.x & 31, tt = tw * 32 + lane;
+    const int CR = 8 * W, CAP = 128 * W;
+    const int r0 = __ldg(q.row0 + un.sys), r1 = __ldg(q.row0 + un.sys + 1), K = __ldg(q.sk + un.sys);
+    const bool lk = lane < un.kc, far = (un.rwlog & 256) != 0;
+    const long long xb = __ldg(q.soff + un.sys) + un.c0 + lane;  // + (row - r0) * K
+    int kp = 1;
+    while (kp < un.kc) kp <<= 1;
+    const int rw = 1 << (un.rwlog & 255), zero = rw * kp;  // the ring's zero row
+    T* ring = reinterpret_cast<T*>(region);
+    double* solb = reinterpret_cast<double*>(region + SeqSmem<T>::ent + tw * SeqSmem<T>::rhs) + lane;
+    BT* rhsb = reinterpret_cast<BT*>(solb - lane + 4 * 32) + lane;  // 32 columns a row, row i in place i & 3
+    SeqEntry<T>* ent = reinterpret_cast<SeqEntry<T>*>(region + SeqSmem<T>::ent + W * SeqSmem<T>::rhs);
+    T* sdi = reinterpret_cast<T*>(ent + 2 * CAP);
+    T* sum = sdi + 2 * CR + tt;  // this lane's sum of a row's early part
+    int* slate = reinterpret_cast<int*>(sdi + 2 * CR + 32 * W);
+    int* rp = slate + 2 * CR;
+    T* mine = ring + (lk ? lane : 0);
+    constexpr int H = 4;  // rows from a row to the one it hands over to early (W = 7)
+    auto team_sync = [&]() {
+        if (W > 1) asm volatile("barrier.cta.sync 15, %0;" ::"r"(32 * W) : "memory");
+        else __syncwarp();
+    };
+    auto ring_at = [&](int r, int c) { return far && r - c >= rw ? ~(c - r0) : (c & (rw - 1)) * kp; };
+    const int nch = (r1 - r0 + CR - 1) / CR;
+    // chunk c's row pointers, and its staged part: a thread's share in registers
+    auto ld_ptr = [&](int c) { return tt <= CR && c < nch ? load_now(q.ptr + min(r0 + c * CR + tt, r1)) : 0; };
+    auto st_ptr = [&](int c, int v) {
+        if (tt <= CR) rp[(c % 3) * (CR + 1) + tt] = v;
+    };
+    int pc[4], pl = 0;
+    T pv[4], pd = (T)0;
+    auto ld_chunk = [&](int c) {
+        const int* p = rp + (c % 3) * (CR + 1);
+        const int s0 = p[0], E = p[CR] - s0;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (E <= CAP && tt + k * 32 * W < E) {
+                pc[k] = load_now(q.col + s0 + tt + k * 32 * W);
+                pv[k] = (T)load_now(val + s0 + tt + k * 32 * W);
+            }
+        if (tt < CR && r0 + c * CR + tt < r1) {
+            pd = (T)load_now(di + r0 + c * CR + tt);
+            pl = load_now(q.late + r0 + c * CR + tt);
+        }
+    };
+    auto st_chunk = [&](int c) {
+        const int* p = rp + (c % 3) * (CR + 1);
+        const int E = p[CR] - p[0], top = min(r0 + (c + 1) * CR, r1);
+        SeqEntry<T>* d = ent + (c & 1) * CAP;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            if (E <= CAP && tt + k * 32 * W < E) {
+                SeqEntry<T> en;
+                en.v = -pv[k];
+                // past the ring for some row of the chunk: read from x for all of them
+                en.at = far && top - pc[k] > rw ? ~(pc[k] - r0) : (pc[k] & (rw - 1)) * kp;
+                d[tt + k * 32 * W] = en;
+            }
+        if (tt < CR) {
+            sdi[(c & 1) * CR + tt] = pd;
+            slate[(c & 1) * CR + tt] = pl;
+        }
+    };
+    // right-hand sides three own rows ahead, each lane its own, by copies that hold no register
+    const long long step = (long long)W * K;
+    T* xo = x + xb + (long long)tw * K;            // this warp's next row of x
+    const BT* bo = b + xb + (long long)tw * K;     // the next row of b to fetch
+    int br = r0 + tw;
+    auto rhs = [&](int i) {
+        if (lk && br < r1) {
+            seq_copy(rhsb + (i & 3) * 32, bo);
+            if (OUT == 2) seq_copy(solb + (i & 3) * 32, x64 + (bo - b));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        br += W;
+        bo += step;
+    };
+    if (tw == 0) ring[zero + lane] = (T)0;
+    st_ptr(0, ld_ptr(0));
+    st_ptr(1, ld_ptr(1));
+    team_sync();
+    ld_chunk(0);
+    st_chunk(0);
+    rhs(0);
+    rhs(1);
+    rhs(2);
+    team_sync();
+    const bool halves = W == 7;
+    const int next = 1 + (tw + 1 == W ? 0 : tw + 1), ahead = 8 + (tw + H) % W;
+    for (int c = 0; c < nch; c++) {
+        if (c + 1 < nch) ld_chunk(c + 1);
+        const int pn = ld_ptr(c + 2);
+        const int* p = rp + (c % 3) * (CR + 1);
+        const int s0 = p[0];
+        const bool staged = p[CR] - s0 <= CAP;
+        const SeqEntry<T>* d = ent + (c & 1) * CAP;
+        const int* late = slate + (c & 1) * CR;
+        const T* dis = sdi + (c & 1) * CR;
+        int i = c * 8;  // own row
+        for (int rr = tw; rr < CR; rr += W, i++) {
+            const int r = r0 + c * CR + rr;
+            if (r >= r1) break;
+            // halfway: the next chunk has landed, and every row of the last one, whose
+            // place it takes, has handed over; it is there for this warp's rows of the next
+            // chunk because the team's rows between hand over one after another
+            if (rr - tw == 4 * W) {
+                if (c + 1 < nch) st_chunk(c + 1);
+                st_ptr(c + 2, pn);
+                if (W == 1) __syncwarp();
+            }
+            const int s = p[rr] - s0, n = p[rr + 1] - s0 - s, cnt = late[rr];
+            const T piv = dis[rr];
+            asm volatile("cp.async.wait_group 2;" ::: "memory");
+            const T b1 = lk ? (T)rhsb[(i & 3) * 32] : (T)0;
+            const double o1 = OUT == 2 && lk ? solb[(i & 3) * 32] : 0.0;
+            rhs(i + 3);
+            const bool turn = W > 1 && r > r0;
+            T* slot = mine + (r & (rw - 1)) * kp;
+            T res;
+            if (staged && !far) {
+                const int nl = cnt & 15, nm = cnt >> 4, ne = n - nl - nm, rem = ne & 3;
+                const SeqEntry<T>* e = d + s;
+                T a0 = b1, a1 = (T)0, a2 = (T)0, a3 = (T)0;
+                for (const SeqEntry<T>* top = e + (ne - rem); e < top; e += 4) {
+                    const SeqEntry<T> e0 = e[0], e1 = e[1], e2 = e[2], e3 = e[3];
+                    const T x0 = mine[e0.at], x1 = mine[e1.at], x2 = mine[e2.at], x3 = mine[e3.at];
+                    a0 += e0.v * x0;
+                    a1 += e1.v * x1;
+                    a2 += e2.v * x2;
+                    a3 += e3.v * x3;
+                }
+                if (rem) {
+                    const SeqEntry<T> e0 = e[0], e1 = e[rem > 1 ? 1 : 0], e2 = e[rem > 2 ? 2 : 0];
+                    const T x0 = mine[e0.at], x1 = mine[e1.at], x2 = mine[e2.at];
+                    a1 += e0.v * x0;
+                    a2 += (rem > 1 ? e1.v : (T)0) * x1;
+                    a3 += (rem > 2 ? e2.v : (T)0) * x2;
+                    e += rem;
+                }
+                if (halves && r - H >= r0) {
+                    if (nm) {
+                        const SeqEntry<T> e0 = e[0], e1 = e[nm > 1 ? 1 : 0], e2 = e[nm > 2 ? 2 : 0];
+                        asm volatile("barrier.cta.sync %0, 64;" ::"r"(8 + tw) : "memory");
+                        const T x0 = mine[e0.at], x1 = mine[e1.at], x2 = mine[e2.at];
+                        a1 += e0.v * x0;
+                        a2 += (nm > 1 ? e1.v : (T)0) * x1;
+                        a3 += (nm > 2 ? e2.v : (T)0) * x2;
+                        e += nm;
+                    } else {  // nothing to wait for
+                        asm volatile("barrier.cta.arrive %0, 64;" ::"r"(8 + tw) : "memory");
+                    }
+                }
+                const T acc = (a0 + a1) + (a2 + a3);
+                if (nl == 0) {
+                    res = acc * piv;
+                    if (lk) *slot = res;
+                    if (turn) asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + tw) : "memory");
+                } else {
+                    const SeqEntry<T> e0 = e[0], e1 = e[nl > 1 ? 1 : 0], e2 = e[nl > 2 ? 2 : 0];
+                    const T v1 = nl > 1 ? e1.v : (T)0, v2 = nl > 2 ? e2.v : (T)0;
+                    *sum = acc;  // through memory, so that its arithmetic is done before the turn
+                    if (turn) asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + tw) : "memory");
+                    const T x0 = mine[e0.at], x1 = mine[e1.at], x2 = mine[e2.at];
+                    T t = *sum;
+                    t += e0.v * x0;
+                    t += v1 * x1;
+                    t += v2 * x2;
+                    res = t * piv;
+                    if (lk) *slot = res;
+                }
+            } else {  // everything in the row's turn
+                if (halves && r - H >= r0) asm volatile("barrier.cta.arrive %0, 64;" ::"r"(8 + tw) : "memory");
+                if (turn) asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + tw) : "memory");
+                T t = b1;
+                for (int k = 0; k < n; k++) {
+                    SeqEntry<T> e;
+                    if (staged) {
+                        e = d[s + k];
+                    } else {
+                        const int cc = __ldg(q.col + s0 + s + k);
+                        e.v = -(T)__ldg(val + s0 + s + k);
+                        e.at = ring_at(r, cc);
+                    }
+                    if (e.at >= 0) t += e.v * mine[e.at];
+                    else if (lk) t += e.v * ld_relaxed(x + xb + (long long)(~e.at) * K);
+                }
+                res = t * piv;
+                if (lk) *slot = res;
+            }
+            if (W > 1 && r + 1 < r1) asm volatile("barrier.cta.arrive %0, 64;" ::"r"(next) : "memory");
+            if (halves && r + H < r1) asm volatile("barrier.cta.arrive %0, 64;" ::"r"(ahead) : "memory");
+            if (lk) {
+                const T pub = publishable(res);
+                *xo = pub;
+                if (OUT == 1) x64[xo - x] = (double)pub;
+                if (OUT == 2) x64[xo - x] = o1 + (double)pub;
+            }
+            xo += step;
+        }
+    }
+    team_sync();  // before the team's next unit
+}
+
+// The other form, for batches with more units than teams can take at once: one
+// warp per unit.  A column a row costs it 255 cycles against a team's 222 for
+// all of them, but 1,184 such warps run at a time against 148 teams.
 __device__ __forceinline__ void cp_async(void* dst, const void* src, int bytes_is8)
 {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
@@ -159,16 +459,21 @@ __device__ __forceinline__ void cp_async(void* dst, const void* src, int bytes_i
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Shared memory of one sequential warp: the ring of recent x values, then
+constexpr int kSweepRing = 1024;       // ring elements of a sweeping warp
+constexpr int kSweepEC = 512;          // entries of one 32-row chunk that fit a stage buffer
+constexpr int kSweepMaxK = 8;          // most right-hand sides one such warp carries
+constexpr int kSweepSplitRows = 16384; // systems this long get one warp per right-hand side
+
+// Shared memory of one sweeping warp: the ring of recent x values, then
 // two stage buffers of one 32-row chunk each (relative row pointers, 1/diag,
 // columns, values, right-hand sides).
 template <typename V, typename T, typename BT>
-struct SeqSmem {
+struct SweepSmem {
     static constexpr size_t al(size_t x) { return (x + 15) & ~size_t(15); }
-    static constexpr size_t ring = al(kSeqRing * sizeof(T));
+    static constexpr size_t ring = al(kSweepRing * sizeof(T));
     static constexpr size_t o_ptr = 0, o_di = al(33 * 4), o_col = o_di + al(32 * sizeof(V)),
-                            o_val = o_col + al(kSeqEC * 4), o_b = o_val + al(kSeqEC * sizeof(V)),
-                            buf = o_b + al(32 * kSeqMaxK * sizeof(BT));
+                            o_val = o_col + al(kSweepEC * 4), o_b = o_val + al(kSweepEC * sizeof(V)),
+                            buf = o_b + al(32 * kSweepMaxK * sizeof(BT));
     static constexpr size_t total = ring + 2 * buf;
 };
 
@@ -182,13 +487,13 @@ struct SeqSmem {
 // owns right-hand side q (all of K > 1 columns, products subtracted in
 // element order), or, for one column, lane j owns row j of each chunk (a
 // sweep; the column's values are strided by K in b and x).  A chunk with
-// more than kSeqEC entries is read from global memory instead.
+// more than kSweepEC entries is read from global memory instead.
 template <typename V, typename T, typename BT, int OUT>
-__device__ __forceinline__ void seq_system(const SeqSet& q, const V* __restrict__ val, const V* __restrict__ di,
+__device__ __forceinline__ void sweep_unit(const SeqSet& q, const V* __restrict__ val, const V* __restrict__ di,
                                            int s, int col, const BT* __restrict__ b, T* x, double* x64,
                                            unsigned char* region)
 {
-    using SM = SeqSmem<V, T, BT>;
+    using SM = SweepSmem<V, T, BT>;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int r0 = __ldg(q.row0 + s), r1 = __ldg(q.row0 + s + 1), K = __ldg(q.sk + s);
@@ -197,7 +502,7 @@ __device__ __forceinline__ void seq_system(const SeqSet& q, const V* __restrict_
     const int c0 = col >= 0 ? col : 0; // first of them
     int kp = 1;
     while (kp < Ke) kp <<= 1;
-    const int rw = kSeqRing / kp;
+    const int rw = kSweepRing / kp;
     const bool lk = lane < K;
     T* ring = reinterpret_cast<T*>(region);
     auto bufp = [&](int bi) { return region + SM::ring + (size_t)bi * SM::buf; };
@@ -222,7 +527,7 @@ __device__ __forceinline__ void seq_system(const SeqSet& q, const V* __restrict_
             cp_async(sdi + lane, di + cb + lane, sizeof(V) == 8);
         }
         if (lane == 0) sptr[cnt] = E;
-        const bool fits = E <= kSeqEC;
+        const bool fits = E <= kSweepEC;
         if (fits)
             for (int p = lane; p < E; p += 32) {
                 cp_async(scol + p, q.col + a + p, 0);
@@ -380,73 +685,146 @@ __device__ __forceinline__ void seq_system(const SeqSet& q, const V* __restrict_
     }
 }
 
+// A level task on its way to its warp, in two stages: its positions and lanes
+// per row; and, per lane, its row's entry range, packed offset and 1 / diag.
+struct VkHead {
+    int base, cnt, kp;
+};
+template <typename T, typename XI>
+struct VkRow {
+    int base, kp, s, len;
+    XI xr;
+    T piv;
+    bool act;
+};
+
 // Variable right-hand-side count, one lane per (row, right-hand side), over
-// level-aligned tasks.  With sequential systems (q.nseqw > 0) the warps are
-// numbered w = (warp in block) * gridDim + block; w < nseqw runs its
-// sequential systems, the others take the level tasks round-robin.
-template <typename V, typename T, typename BT, int OUT>
-__global__ void __launch_bounds__(512, 1) k_sptrsv_vk(BatchMat bm, const V* __restrict__ val, const V* __restrict__ di,
+// level-aligned tasks.  The dependent loads of a task (positions, rows,
+// the first kVkAhead entries) are issued a stage each during the tasks before
+// it, so once the rows it reads are there it only gathers, kVkU at a time
+// (64 systems of band 700-1500: 9.6 -> 8.4 ms; loaded on the spot, a task's
+// second eight entries came after the first eight's wait).
+// With sequential systems (q.nteams > 0) the first `team` warps of block
+// c < nteams are team c and run its units (SWEEP: warp w = (warp in block) *
+// gridDim + block < nteams runs its own); the other warps take the level tasks
+// round-robin.  XI: packed offsets, 32-bit where they fit.
+template <typename V, typename T, typename BT, int OUT, typename XI, bool SWEEP>
+__global__ void __launch_bounds__(512, 1) k_sptrsv_vk(BatchMat<XI> bm, const V* __restrict__ val, const V* __restrict__ di,
                                                    int ntasks, const int* __restrict__ tbase,
-                                                   const int* __restrict__ tkp, SeqSet q, const V* __restrict__ nval,
-                                                   const V* __restrict__ ndi, const BT* __restrict__ b, T* x,
-                                                   double* x64, DevStatus* st, unsigned long long budget,
-                                                   unsigned backoff)
+                                                   const int* __restrict__ tkp, SeqSet q, int team,
+                                                   const V* __restrict__ nval, const V* __restrict__ ndi,
+                                                   const BT* __restrict__ b, T* x, double* x64, DevStatus* st,
+                                                   unsigned long long budget, unsigned backoff)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int w = wib * (int)gridDim.x + (int)blockIdx.x;
-    if (w < q.nseqw) {  // w < nseqw implies wib < the sequential warps per block, each with its region
-        for (int z = __ldg(q.wptr + w); z < __ldg(q.wptr + w + 1); z++)
-            seq_system<V, T, BT, OUT>(q, nval, ndi, __ldg(q.wsys + z), __ldg(q.wcol + z), b, x, x64,
-                                      smem_raw + (size_t)wib * SeqSmem<V, T, BT>::total);
-        return;
-    }
-    const int gw = w - q.nseqw;
-    const int nw = (int)(((long long)gridDim.x * blockDim.x) >> 5) - q.nseqw;
-    for (int t = gw; t < ntasks; t += nw) {
-        const int base = __ldg(tbase + t), cnt = __ldg(tbase + t + 1) - base, kp = __ldg(tkp + t);
-        const int seg = lane / kp, k = lane & (kp - 1);
-        const int pos = base + seg;
-        const bool act = seg < cnt && k < __ldg(bm.krow + (seg < cnt ? pos : base));
-        long long xr = 0;
-        T acc = 0, piv = 0;
-        int s = 0, len = 0;
-        double old64 = 0.0;  // the solution a correction adds to, loaded with the task
-        if (act) {
-            xr = __ldg(bm.xrow + pos);
-            acc = (T)b[xr + k];
-            if (OUT == 2) old64 = x64[xr + k];
-            piv = (T)__ldg(di + pos);
-            s = __ldg(bm.ptr + pos);
-            len = __ldg(bm.ptr + pos + 1) - s;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, nwb = blockDim.x >> 5;
+    const int bid = blockIdx.x, nteams = q.nteams;
+    int nw, gw;  // level warps, and this one's number
+    if constexpr (SWEEP) {
+        const int w = wib * (int)gridDim.x + bid;
+        if (w < nteams) {
+            for (int z = __ldg(q.tptr + w); z < __ldg(q.tptr + w + 1); z++)
+                sweep_unit<V, T, BT, OUT>(q, nval, ndi, q.units[z].sys, q.units[z].c0, b, x, x64,
+                                          smem_raw + (size_t)wib * SweepSmem<V, T, BT>::total);
+            return;
         }
+        nw = (int)gridDim.x * nwb - nteams;
+        gw = w - nteams;
+    } else {
+        if (bid < nteams && wib < team) {
+            for (int z = __ldg(q.tptr + bid); z < __ldg(q.tptr + bid + 1); z++)
+                seq_unit<V, T, BT, OUT>(q, nval, ndi, q.units[z], team, wib, b, x, x64, smem_raw);
+            return;
+        }
+        // nwb - team level warps in the first nteams blocks, nwb in the others
+        nw = (int)gridDim.x * nwb - nteams * team;
+        gw = bid < nteams ? bid * (nwb - team) + wib - team : nteams * (nwb - team) + (bid - nteams) * nwb + wib;
+    }
+    auto head = [&](VkHead& h, long long t) {
+        h.base = h.cnt = 0;
+        h.kp = 32;
+        if (t < ntasks) {
+            h.base = __ldg(tbase + t);
+            h.cnt = __ldg(tbase + t + 1) - h.base;
+            h.kp = __ldg(tkp + t);
+        }
+    };
+    auto rows = [&](VkRow<T, XI>& z, const VkHead& h) {
+        const int seg = lane / h.kp, k = lane & (h.kp - 1), pos = h.base + seg;
+        z.base = h.base;
+        z.kp = h.kp;
+        z.s = z.len = 0;
+        z.xr = 0;
+        z.piv = (T)0;
+        z.act = seg < h.cnt && k < __ldg(bm.krow + pos);
+        if (z.act) {
+            z.xr = (XI)__ldg(bm.xrow + pos) + k;
+            z.piv = (T)__ldg(di + pos);
+            z.s = __ldg(bm.ptr + pos);
+            z.len = __ldg(bm.ptr + pos + 1) - z.s;
+        }
+    };
+    XI xc[kVkAhead];
+    T vv[kVkAhead], bn = (T)0;
+    double on = 0.0;
+    auto entries = [&](const VkRow<T, XI>& z, int j) {
+        const int k = lane & (z.kp - 1);
+#pragma unroll
+        for (int u = 0; u < kVkAhead; u++) {
+            xc[u] = 0;
+            vv[u] = (T)0;
+            if (j + u < z.len) {
+                xc[u] = __ldg(bm.xdep + z.s + j + u) + k;
+                vv[u] = (T)__ldg(val + z.s + j + u);
+            }
+        }
+    };
+    auto rhs = [&](const VkRow<T, XI>& z) {
+        bn = z.act ? (T)b[z.xr] : (T)0;
+        if (OUT == 2) on = z.act ? x64[z.xr] : 0.0;  // the solution a correction adds to
+    };
+    VkHead h;
+    VkRow<T, XI> cur, nxt;
+    head(h, gw);
+    rows(cur, h);
+    head(h, gw + (long long)nw);
+    rows(nxt, h);
+    head(h, gw + 2LL * nw);
+    entries(cur, 0);
+    rhs(cur);
+    for (long long t = gw; t < ntasks; t += nw) {
+        T acc = bn;
+        const double old64 = on;
         // rows of a task are in one level: the warp waits for each round of
         // kVkU elements together (loads issued back to back)
-        const int rounds = __reduce_max_sync(0xffffffffu, len);
-        for (int j = 0; j < rounds; j += kVkU) {
-            const int nh = min(kVkU, len - j);
-            long long xc[kVkU];
-            T vv[kVkU], xv[kVkU];
+        const int rounds = __reduce_max_sync(0xffffffffu, cur.len);
+        for (int j = 0; j < rounds; j += kVkAhead) {
+            if (j > 0) entries(cur, j);
 #pragma unroll
-            for (int u = 0; u < kVkU; u++) {
-                xc[u] = 0;
-                vv[u] = 0;
-                if (u < nh) {
-                    xc[u] = __ldg(bm.xdep + s + j + u) + k;
-                    vv[u] = (T)__ldg(val + s + j + u);
-                }
+            for (int h2 = 0; h2 < kVkAhead; h2 += kVkU) {
+                if (h2 > 0 && j + h2 >= rounds) break;
+                XI xq[kVkU];
+                T xv[kVkU];
+#pragma unroll
+                for (int u = 0; u < kVkU; u++) xq[u] = xc[h2 + u];
+                const int nh = min(kVkU, cur.len - j - h2);
+                if (!warp_wait_n<false, kVkU, T>(nh, xq, x, nullptr, xv, st, budget, backoff, cur.base)) return;
+#pragma unroll
+                for (int u = 0; u < kVkU; u++)
+                    if (u < nh) acc -= vv[h2 + u] * xv[u];
             }
-            if (!warp_wait_n<false, kVkU, T>(nh, xc, x, nullptr, xv, st, budget, backoff, pos)) return;
-#pragma unroll
-            for (int u = 0; u < kVkU; u++)
-                if (u < nh) acc -= vv[u] * xv[u];
         }
-        if (act) {
-            T r = publishable(acc * piv);
-            st_relaxed(x + xr + k, r);
-            if (OUT == 1) x64[xr + k] = (double)r;
-            if (OUT == 2) x64[xr + k] = old64 + (double)r;
+        if (cur.act) {
+            T r = publishable(acc * cur.piv);
+            st_relaxed(x + cur.xr, r);
+            if (OUT == 1) x64[cur.xr] = (double)r;
+            if (OUT == 2) x64[cur.xr] = old64 + (double)r;
         }
+        cur = nxt;
+        entries(cur, 0);
+        rhs(cur);
+        rows(nxt, h);
+        head(h, t + 3LL * nw);
     }
 }
 
@@ -607,12 +985,13 @@ __global__ void k_batch_rows(const int* __restrict__ order, const int* __restric
 }
 
 // level layout positions p < n_lvl from the natural-order union
+template <typename XI>
 __global__ void k_batch_fill(const int* __restrict__ order, const int* __restrict__ nptr, const int* __restrict__ ncol,
                              const double* __restrict__ nval, const double* __restrict__ ndg,
                              const int* __restrict__ sys_of_row, const int* __restrict__ row0,
                              const long long* __restrict__ soff, const int* __restrict__ sk,
                              const int* __restrict__ ptr, int n_lvl, long long* __restrict__ xrow,
-                             int* __restrict__ krow, long long* __restrict__ xdep, double* __restrict__ val64,
+                             int* __restrict__ krow, XI* __restrict__ xdep, double* __restrict__ val64,
                              float* __restrict__ val32, double* __restrict__ dg64, double* __restrict__ di64,
                              float* __restrict__ di32)
 {
@@ -626,7 +1005,7 @@ __global__ void k_batch_fill(const int* __restrict__ order, const int* __restric
         const int a = nptr[r], e = nptr[r + 1], dst = ptr[p];
         for (int q = a + lane; q < e; q += 32) {
             const int c = ncol[q];
-            xdep[dst + q - a] = o + (long long)(c - r0) * k;
+            xdep[dst + q - a] = (XI)(o + (long long)(c - r0) * k);
             val64[dst + q - a] = nval[q];
             val32[dst + q - a] = (float)nval[q];
         }
@@ -638,6 +1017,19 @@ __global__ void k_batch_fill(const int* __restrict__ order, const int* __restric
             di64[p] = 1.0 / d;
             di32[p] = 1.0f / (float)d;
         }
+    }
+}
+
+// entries of each row that its team's warp takes late (columns ascend): the
+// ones less than W rows back, or with 7 warps the ones less than 4 back, and
+// 16 times those 4 to 6 back
+__global__ void k_late(const int* __restrict__ nptr, const int* __restrict__ ncol, int n, int W,
+                       unsigned char* __restrict__ late)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int k = 0;
+        for (int p = nptr[i + 1] - 1; p >= nptr[i] && ncol[p] > i - W; p--) k += W == 7 && ncol[p] <= i - 4 ? 16 : 1;
+        late[i] = (unsigned char)k;
     }
 }
 
@@ -763,13 +1155,15 @@ void batch_free(sptrsv_batch_s* B)
     cudaFree(B->nptr); cudaFree(B->ncol); cudaFree(B->nval64); cudaFree(B->nval32); cudaFree(B->ndg64);
     cudaFree(B->ndi64); cudaFree(B->ndi32); cudaFree(B->tsys); cudaFree(B->tj); cudaFree(B->cdep);
     cudaFree(B->sys_row0); cudaFree(B->sys_chunk0); cudaFree(B->sys_k); cudaFree(B->sys_off); cudaFree(B->flags);
-    cudaFree(B->row_sys); cudaFree(B->lev); cudaFree(B->d_kplog); cudaFree(B->wptr); cudaFree(B->wsys);
-    cudaFree(B->wcol);
+    cudaFree(B->row_sys); cudaFree(B->lev); cudaFree(B->d_kplog); cudaFree(B->tptr); cudaFree(B->units); cudaFree(B->late);
     cudaFree(B->rblk_sys); cudaFree(B->rblk_e0);
     cudaFree(B->ptr); cudaFree(B->xrow); cudaFree(B->krow); cudaFree(B->xdep); cudaFree(B->val64);
     cudaFree(B->val32); cudaFree(B->dg64); cudaFree(B->di64); cudaFree(B->di32); cudaFree(B->tbase);
     cudaFree(B->tkp); cudaFree(B->w32a); cudaFree(B->w32b);
 }
+
+// Packed offsets past 32 bits.
+bool wide_offsets(const sptrsv_batch_s* B) { return B->nvec > 0xffffffffLL; }
 
 // Level- and class-aligned tasks over the first n_lvl layout positions: a
 // segment is one (level, kp) key and is cut into tasks of 32/kp rows;
@@ -797,7 +1191,8 @@ int batch_level_layout(sptrsv_batch_s* B, cudaStream_t s)
     }
     cudaFree(B->xrow); cudaFree(B->xdep); cudaFree(B->val64); cudaFree(B->val32); cudaFree(B->dg64);
     cudaFree(B->di64); cudaFree(B->di32);
-    B->xrow = B->xdep = nullptr;
+    B->xrow = nullptr;
+    B->xdep = nullptr;
     B->val64 = B->dg64 = B->di64 = nullptr;
     B->val32 = B->di32 = nullptr;
     B->ntasks = 0;
@@ -840,17 +1235,21 @@ int batch_level_layout(sptrsv_batch_s* B, cudaStream_t s)
     m_lvl = mm;
     LCHK(dalloc(&B->xrow, n_lvl));
     LCHK(dalloc(&B->krow, n_lvl));
-    LCHK(dalloc(&B->xdep, m_lvl));
+    LCHK(cudaMalloc(&B->xdep, (wide_offsets(B) ? 8 : 4) * (size_t)std::max<long long>(1, m_lvl)));
     LCHK(dalloc(&B->val64, m_lvl));
     LCHK(dalloc(&B->val32, m_lvl));
     LCHK(dalloc(&B->dg64, n_lvl));
     LCHK(dalloc(&B->di64, n_lvl));
     LCHK(dalloc(&B->di32, n_lvl));
     if (n_lvl > 0) {
-        k_batch_fill<<<grid_for(n_lvl * 32, 256), 256, 0, s>>>(ord, B->nptr, B->ncol, B->nval64, B->ndg64,
-                                                                B->row_sys, B->sys_row0, B->sys_off, B->sys_k,
-                                                                B->ptr, (int)n_lvl, B->xrow, B->krow, B->xdep,
-                                                                B->val64, B->val32, B->dg64, B->di64, B->di32);
+        auto fill = [&](auto* xdep) {
+            k_batch_fill<<<grid_for(n_lvl * 32, 256), 256, 0, s>>>(ord, B->nptr, B->ncol, B->nval64, B->ndg64,
+                                                                    B->row_sys, B->sys_row0, B->sys_off, B->sys_k,
+                                                                    B->ptr, (int)n_lvl, B->xrow, B->krow, xdep,
+                                                                    B->val64, B->val32, B->dg64, B->di64, B->di32);
+        };
+        if (wide_offsets(B)) fill(static_cast<long long*>(B->xdep));
+        else fill(static_cast<unsigned*>(B->xdep));
         LCHK(cudaGetLastError());
     }
     {
@@ -868,118 +1267,161 @@ int batch_level_layout(sptrsv_batch_s* B, cudaStream_t s)
 
 constexpr int kModeLevel = 0, kModeChunk = 1, kModeHybrid = 2;
 constexpr double kSeqAll = 1e9;  // a sequential width this large makes every system sequential
-constexpr int kSeqSplitRows = 16384;  // sequential systems this long get one warp per right-hand side
 
-// Sequential warps per block (warps 0.. of each block), each with its own
-// shared-memory region; the other warps take the level tasks.
-int seq_per_block(const sptrsv_batch_s* B) { return B->block_warps >= 8 ? 4 : B->block_warps >= 4 ? 2 : 1; }
+// Warps of a block's sequential team (warps 0.. of the block, one ring); the
+// other warps take the level tasks.
+int seq_team(const sptrsv_batch_s* B) { return B->block_warps >= 8 ? 7 : B->block_warps / 2; }
 
+// Warps per block of the level-ordered launch: a team needs as many again for
+// the level tasks.
+int vk_warps(const sptrsv_batch_s* B, bool teams) { return teams && B->block_warps == 8 ? 16 : B->block_warps; }
+// Sweeping warps per block.
+int sweep_per_block(const sptrsv_batch_s* B) { return B->block_warps >= 8 ? 4 : B->block_warps >= 4 ? 2 : 1; }
 
 // The level-ordered launch's grid size (every instantiation that a solve
-// launches), before any sequential-warp assignment.
+// launches), before any sequential-team assignment.
 template <typename V, typename T, typename BT, int OUT>
-int vk_grid(const sptrsv_batch_s* B, long long max_blocks, long long* g)
+int vk_grid(const sptrsv_batch_s* B, bool sweep, long long max_blocks, long long* g)
 {
-    const int cap = B->warps_per_sm > 0 ? (B->warps_per_sm + B->block_warps - 1) / B->block_warps : 0;
-    const size_t smem = (size_t)seq_per_block(B) * SeqSmem<V, T, BT>::total;
-    auto kern = k_sptrsv_vk<V, T, BT, OUT>;
-    if (smem > 32 * 1024)  // the occupancy query needs the kernel's opt-in to large shared memory
-        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SPT_CUDA(persistent_grid(kern, 32 * B->block_warps, smem, max_blocks, cap, g));
-    return 0;
+    const int bw = sweep ? B->block_warps : vk_warps(B, true);
+    const int cap = B->warps_per_sm > 0 ? (B->warps_per_sm + bw - 1) / bw : 0;
+    const size_t smem = sweep ? sweep_per_block(B) * SweepSmem<V, T, BT>::total : SeqSmem<T>::total(seq_team(B));
+    auto grid = [&](auto kern) -> int {
+        if (smem > 32 * 1024)  // the occupancy query needs the kernel's opt-in to large shared memory
+            SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SPT_CUDA(persistent_grid(kern, 32 * bw, smem, max_blocks, cap, g));
+        return 0;
+    };
+    if (sweep)
+        return wide_offsets(B) ? grid(k_sptrsv_vk<V, T, BT, OUT, long long, true>)
+                               : grid(k_sptrsv_vk<V, T, BT, OUT, unsigned, true>);
+    return wide_offsets(B) ? grid(k_sptrsv_vk<V, T, BT, OUT, long long, false>)
+                           : grid(k_sptrsv_vk<V, T, BT, OUT, unsigned, false>);
 }
 
-long long vk_max_blocks(const sptrsv_batch_s* B, int nseqw)
+// The smallest grid among the instantiations that a solve launches.
+int vk_min_grid(const sptrsv_batch_s* B, bool sweep, long long max_blocks, long long* gmin)
 {
-    const long long a = div_up(B->ntasks, B->block_warps), c = div_up(nseqw, seq_per_block(B));
-    return std::max(std::max(a, c), 1LL);
+    long long g[3] = {};
+    int e = vk_grid<double, double, double, 0>(B, sweep, max_blocks, g);
+    if (!e) e = vk_grid<float, float, double, 1>(B, sweep, max_blocks, g + 1);
+    if (!e) e = vk_grid<float, float, float, 2>(B, sweep, max_blocks, g + 2);
+    *gmin = std::min(g[0], std::min(g[1], g[2]));
+    return e;
+}
+
+long long vk_max_blocks(const sptrsv_batch_s* B, bool sweep, int nteams)
+{
+    if (nteams == 0) return std::max(div_up(B->ntasks, B->block_warps), 1);
+    if (sweep) return std::max(std::max(div_up(B->ntasks, B->block_warps), div_up(nteams, sweep_per_block(B))), 1);
+    const int lw = vk_warps(B, true) - seq_team(B);  // level warps of a block
+    return std::max(std::max(div_up(B->ntasks, lw), nteams), 1);
+}
+
+// Spreads units (of `work` each) over at most nt teams, longest first, each to
+// the team with the least work so far; returns the largest team's work.
+template <class F>
+double spread_units(const std::vector<SeqUnit>& list, int nt, F&& work, std::vector<SeqUnit>& out, std::vector<int>& tp)
+{
+    std::vector<SeqUnit> sorted(list);
+    std::stable_sort(sorted.begin(), sorted.end(), [&](const SeqUnit& a, const SeqUnit& b) { return work(a) > work(b); });
+    std::vector<std::vector<SeqUnit>> per(nt);
+    std::vector<std::pair<double, int>> heap;  // smallest load first
+    for (int w = 0; w < nt; w++) heap.push_back({0.0, w});
+    auto later = [](const std::pair<double, int>& a, const std::pair<double, int>& b) { return a > b; };
+    double top = 0;
+    for (const SeqUnit& u : sorted) {
+        std::pop_heap(heap.begin(), heap.end(), later);
+        per[heap.back().second].push_back(u);
+        heap.back().first += work(u);
+        top = std::max(top, heap.back().first);
+        std::push_heap(heap.begin(), heap.end(), later);
+    }
+    out.clear();
+    tp.assign(nt + 1, 0);
+    for (int w = 0; w < nt; w++) {
+        out.insert(out.end(), per[w].begin(), per[w].end());
+        tp[w + 1] = (int)out.size();
+    }
+    return top;
 }
 
 // Marks the sequential systems (mode 2: n_s / nlevs_s < seq_width and every
-// dependency within the ring window: kSeqRing / kp rows, or kSeqRing rows for
-// a system with more than kSeqMaxK right-hand sides or of at least
-// kSeqSplitRows rows and several right-hand sides, which is solved one column
-// per warp; or every system when seq_width >= kSeqAll),
-// rebuilds the level layout when
-// the set changed, and spreads the sequential systems
-// over at most seq_per_block warps per block of the grid, largest first, each to the warp
-// with the least work so far.
+// dependency at most kSeqMaxDist rows back; or every system when seq_width >=
+// kSeqAll), rebuilds the level layout when the set changed, and spreads the
+// systems over teams: units of as many columns as a ring over their reach
+// holds, one team a block; or, when the longest team is shorter so, over single
+// warps (the measured cycles a row of each form decide).
 int batch_apply_schedule(sptrsv_batch_s* B, cudaStream_t s)
 {
     std::vector<char> seq(B->nsys, 0);
     if (B->mode == kModeHybrid)
         for (int k = 0; k < B->nsys; k++) {
             const double nk = B->row0h[k + 1] - B->row0h[k];
-            int kp = 1;
-            while (kp < B->kk[k]) kp <<= 1;
-            // a split system's units carry one column each: their ring spans kSeqRing rows
-            const bool split = B->kk[k] > kSeqMaxK || (B->kk[k] > 1 && nk >= kSeqSplitRows);
-            const bool fits = B->sys_dist[k] <= (split ? kSeqRing : kSeqRing / kp);
-            seq[k] = B->seq_width >= kSeqAll || (fits && nk < B->seq_width * std::max(1, B->sys_nlev[k]));
+            seq[k] = B->seq_width >= kSeqAll ||
+                     (B->sys_dist[k] <= kSeqMaxDist && nk < B->seq_width * std::max(1, B->sys_nlev[k]));
         }
     if (seq != B->seq || !B->ptr) {
         B->seq = seq;
         int e = batch_level_layout(B, s);
         if (e) return e;
     }
-    // units: a system with more than kSeqMaxK right-hand sides, or a long one
-    // with several, becomes one unit per column (each swept by its own warp,
-    // 0.13 us per row on a near-chain); other systems are one unit carrying
-    // all their columns (0.4 us per row for K > 1)
-    std::vector<std::pair<int, int>> list;
+    std::vector<SeqUnit> teams, sweeps;
     for (int k = 0; k < B->nsys; k++) {
         if (!B->seq[k]) continue;
+        int rwlog = 5, kp = 1;
+        while (kp < B->kk[k]) kp <<= 1;
+        const int need = B->sys_dist[k] + 8;  // its reach, and the rows in the team's hands
         const int nk = B->row0h[k + 1] - B->row0h[k];
-        if (B->kk[k] > kSeqMaxK || (B->kk[k] > 1 && nk >= kSeqSplitRows))
-            for (int c = 0; c < B->kk[k]; c++) list.push_back({k, c});
+        if (B->kk[k] > kSweepMaxK || (B->kk[k] > 1 && (nk >= kSweepSplitRows || B->sys_dist[k] > kSweepRing / kp)))
+            for (int c = 0; c < B->kk[k]; c++) sweeps.push_back({k, c, 1, 0});
         else
-            list.push_back({k, -1});
+            sweeps.push_back({k, -1, B->kk[k], 0});
+        while ((1 << rwlog) < need && (2 << rwlog) * 4 <= kSeqElems) rwlog++;  // at least 4 columns
+        const bool far = (1 << rwlog) < need;
+        while ((kp << rwlog) > kSeqElems) kp >>= 1;
+        for (int c = 0; c < B->kk[k]; c += kp)
+            teams.push_back({k, c, std::min(kp, B->kk[k] - c), rwlog | (far ? 256 : 0)});
     }
-    cudaFree(B->wptr);
-    cudaFree(B->wsys);
-    cudaFree(B->wcol);
-    B->wptr = B->wsys = B->wcol = nullptr;
-    B->nseqw = 0;
-    if (list.empty()) return 0;
-    long long g = 0, gmin = 1LL << 40;
-    const long long mb = vk_max_blocks(B, (int)list.size());
-    int e = vk_grid<double, double, double, 0>(B, mb, &g);
-    if (e) return e;
-    gmin = std::min(gmin, g);
-    if ((e = vk_grid<float, float, double, 1>(B, mb, &g))) return e;
-    gmin = std::min(gmin, g);
-    if ((e = vk_grid<float, float, float, 2>(B, mb, &g))) return e;
-    gmin = std::min(gmin, g);
-    const int nw = (int)std::min<long long>((long long)list.size(), gmin * seq_per_block(B));
-    auto work = [&](const std::pair<int, int>& u) {
-        const double nk = B->row0h[u.first + 1] - B->row0h[u.first];
-        return nk * (u.second >= 0 || B->kk[u.first] == 1 ? 1.0 : 3.0);
-    };
-    std::stable_sort(list.begin(), list.end(), [&](const std::pair<int, int>& a, const std::pair<int, int>& b2) {
-        return work(a) > work(b2);
-    });
-    std::vector<std::vector<std::pair<int, int>>> per(nw);
-    std::vector<double> load(nw, 0.0);
-    for (const auto& u : list) {
-        const int w = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        per[w].push_back(u);
-        load[w] += work(u);
+    cudaFree(B->tptr);
+    cudaFree(B->units);
+    B->tptr = B->units = nullptr;
+    B->nteams = 0;
+    B->sweep = false;
+    if (teams.empty()) return 0;
+    const int W = seq_team(B);
+    std::vector<SeqUnit> list[2];
+    std::vector<int> tp[2];
+    double top[2];
+    int nt[2];
+    for (int f = 0; f < 2; f++) {
+        const std::vector<SeqUnit>& units = f ? sweeps : teams;
+        const int most = (int)std::min<size_t>(units.size(), 1u << 20);
+        long long g = 0;
+        int e = vk_min_grid(B, f != 0, vk_max_blocks(B, f != 0, most), &g);
+        if (e) return e;
+        nt[f] = (int)std::min<long long>(most, f ? g * sweep_per_block(B) : g);
+        // cycles a row: a team of 7, 2 or 1 warps; one warp sweeping one column, or carrying several
+        const double row = f ? 255 : W == 7 ? 222 : W == 2 ? 700 : 1300;
+        auto work = [&](const SeqUnit& u) {
+            return (double)(B->row0h[u.sys + 1] - B->row0h[u.sys]) * (f && u.c0 < 0 && u.kc > 1 ? 750 : row);
+        };
+        top[f] = spread_units(units, nt[f], work, list[f], tp[f]);
     }
-    std::vector<int> wp(nw + 1, 0), ws, wc;
-    for (int w = 0; w < nw; w++) {
-        for (const auto& u : per[w]) {
-            ws.push_back(u.first);
-            wc.push_back(u.second);
-        }
-        wp[w + 1] = (int)ws.size();
+    const int f = top[1] < top[0] ? 1 : 0;
+    B->sweep = f != 0;
+    if (!B->sweep && B->late_w != W) {
+        if (!B->late) SPT_CUDA(dalloc(&B->late, B->n));
+        k_late<<<grid_for(B->n, 256), 256, 0, s>>>(B->nptr, B->ncol, B->n, W, B->late);
+        SPT_CUDA(cudaGetLastError());
+        SPT_CUDA(cudaStreamSynchronize(s));
+        B->late_w = W;
     }
-    SPT_CUDA(dalloc(&B->wptr, nw + 1));
-    SPT_CUDA(dalloc(&B->wsys, (long long)ws.size()));
-    SPT_CUDA(dalloc(&B->wcol, (long long)wc.size()));
-    SPT_CUDA(cudaMemcpy(B->wptr, wp.data(), sizeof(int) * wp.size(), cudaMemcpyHostToDevice));
-    SPT_CUDA(cudaMemcpy(B->wsys, ws.data(), sizeof(int) * ws.size(), cudaMemcpyHostToDevice));
-    SPT_CUDA(cudaMemcpy(B->wcol, wc.data(), sizeof(int) * wc.size(), cudaMemcpyHostToDevice));
-    B->nseqw = nw;
+    SPT_CUDA(dalloc(&B->tptr, nt[f] + 1));
+    SPT_CUDA(dalloc(&B->units, 4LL * (long long)list[f].size()));
+    SPT_CUDA(cudaMemcpy(B->tptr, tp[f].data(), sizeof(int) * tp[f].size(), cudaMemcpyHostToDevice));
+    SPT_CUDA(cudaMemcpy(B->units, list[f].data(), sizeof(SeqUnit) * list[f].size(), cudaMemcpyHostToDevice));
+    B->nteams = nt[f];
     return 0;
 }
 
@@ -1007,17 +1449,30 @@ int batch_launch(sptrsv_batch_s* B, bool f32, const BT* b, T* x, double* x64, cu
     const V* di = f32 ? reinterpret_cast<const V*>(B->di32) : reinterpret_cast<const V*>(B->di64);
     const V* nval = f32 ? reinterpret_cast<const V*>(B->nval32) : reinterpret_cast<const V*>(B->nval64);
     const V* ndi = f32 ? reinterpret_cast<const V*>(B->ndi32) : reinterpret_cast<const V*>(B->ndi64);
-    BatchMat bm{B->ptr, B->xrow, B->krow, B->xdep};
-    SeqSet q{B->nptr, B->ncol, B->sys_row0, B->sys_k, B->sys_off, B->wptr, B->wsys, B->wcol, B->nseqw};
-    auto kern = k_sptrsv_vk<V, T, BT, OUT>;
-    const size_t smem = B->nseqw > 0 ? (size_t)seq_per_block(B) * SeqSmem<V, T, BT>::total : 0;
-    if (smem > 32 * 1024)
-        SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    if (B->ntasks == 0 && B->nseqw == 0) return 0;
-    SPT_CUDA(launch_persistent_capped(kern, block, smem, vk_max_blocks(B, B->nseqw), cap, s, bm, val, di, B->ntasks,
-                                      (const int*)B->tbase, (const int*)B->tkp, q, nval, ndi, b, x, x64,
-                                      c->d_status, wait_budget_ns(), (unsigned)B->backoff_ns));
-    return 0;
+    SeqSet q{B->nptr, B->ncol, B->sys_row0, B->sys_k, B->sys_off, B->late, B->tptr, reinterpret_cast<const SeqUnit*>(B->units),
+             B->nteams};
+    const int team = seq_team(B);
+    const size_t smem = B->nteams == 0 ? 0
+                        : B->sweep     ? sweep_per_block(B) * SweepSmem<V, T, BT>::total
+                                       : SeqSmem<T>::total(team);
+    if (B->ntasks == 0 && B->nteams == 0) return 0;
+    const int bw = B->sweep ? B->block_warps : vk_warps(B, B->nteams > 0);
+    const int vcap = B->warps_per_sm > 0 ? (B->warps_per_sm + bw - 1) / bw : 0;
+    auto go = [&](auto kern, auto bm) -> int {
+        if (smem > 32 * 1024)
+            SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SPT_CUDA(launch_persistent_capped(kern, 32 * bw, smem, vk_max_blocks(B, B->sweep, B->nteams), vcap, s, bm, val,
+                                          di, B->ntasks, (const int*)B->tbase, (const int*)B->tkp, q, team, nval, ndi,
+                                          b, x, x64, c->d_status, wait_budget_ns(), (unsigned)B->backoff_ns));
+        return 0;
+    };
+    const BatchMat<unsigned> b32{B->ptr, B->xrow, B->krow, static_cast<const unsigned*>(B->xdep)};
+    const BatchMat<long long> b64{B->ptr, B->xrow, B->krow, static_cast<const long long*>(B->xdep)};
+    if (B->sweep)
+        return wide_offsets(B) ? go(k_sptrsv_vk<V, T, BT, OUT, long long, true>, b64)
+                               : go(k_sptrsv_vk<V, T, BT, OUT, unsigned, true>, b32);
+    return wide_offsets(B) ? go(k_sptrsv_vk<V, T, BT, OUT, long long, false>, b64)
+                           : go(k_sptrsv_vk<V, T, BT, OUT, unsigned, false>, b32);
 }
 
 int batch_residual(sptrsv_batch_s* B, const double* b, const double* x, cudaStream_t s)
@@ -1386,7 +1841,7 @@ int sptrsv_batch_seq_systems(sptrsv_batch_t B, int* nseq, int* nseq_warps, int* 
         int c = 0;
         for (char f : B->seq) c += f ? 1 : 0;
         if (nseq) *nseq = c;
-        if (nseq_warps) *nseq_warps = B->nseqw;
+        if (nseq_warps) *nseq_warps = B->nteams * (B->sweep ? 1 : seq_team(B));
         if (n_level_rows) *n_level_rows = B->n_lvl;
         return ok();
     });
