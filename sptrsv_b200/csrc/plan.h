@@ -77,6 +77,28 @@ struct WaveLayout {
     int maxe = 0;                      // most entries of one slot
 };
 
+// WAVE for block systems of 2D stencils (wave4.cuh, built in strip.cu; null
+// arrays: the matrix takes WaveLayout).
+struct Wave4Layout {
+    double* inv64 = nullptr;   // [nch * 128] 1 / diagonal
+    float* inv32 = nullptr;
+    double* lsub64 = nullptr;  // [nch * 128] L(i, i-1), 0 for a line's first row
+    float* lsub32 = nullptr;
+    double* ev64 = nullptr;    // [nch * 128] the entry outside the line
+    float* ev32 = nullptr;
+    int* ecol = nullptr;       // [nch * 128] its place in xp, or ~place in the group's shared memory
+    int* chunk = nullptr;      // [nch * 4] first row, rows, first place, place in xp (-1: no other group reads it)
+    int* runc = nullptr;       // as in WaveLayout
+    int* grun = nullptr;
+    int* grow = nullptr;
+    int* gseq = nullptr;
+    int* gmap = nullptr;       // [ngroups * 2] as WaveLayout's ghx
+    int ngroups = 0, G = 0;
+    int places = 0;            // most of one group in shared memory
+    double* xp = nullptr;      // [npub] the chunks that another group reads (FP32 solves: as floats)
+    int npub = 0;
+};
+
 // Multi-RHS task table for kp = 1 << j lanes per row (built on demand, see
 // mrhs.cu): 8 ints per task (MrhsTask), level-aligned, each level's pieces of
 // long rows first, then its groups of short rows.
@@ -151,6 +173,7 @@ struct sptrsv_plan_s {
     StripLayout strip;           // STRIP layout (built on demand)
     int row_strip_R = 0;         // R the strip layout was built for (0: none)
     WaveLayout wave;             // WAVE layout (built on demand)
+    Wave4Layout wave4;           // or this one
     // streamed host solves (WAVE, FP64): b copied in segments on a side
     // stream while the kernel runs, one flag word per segment
     int* bflag = nullptr;        // [nseg] epoch of the last copy of each segment
@@ -201,6 +224,9 @@ void strip_free(StripLayout& t);
 // max_rows.
 int build_wave_layout(sptrsv_plan_s* p, int G, int max_rows);
 void wave_free(WaveLayout& w);
+void wave4_free(Wave4Layout& w);
+// Is the plan's WAVE schedule for G lines per CTA built, in either layout?
+bool wave_built(const sptrsv_plan_s* p, int G);
 // Builds (or keeps) the multi-RHS task table for kp lanes per row.
 int build_mrhs_tasks(sptrsv_plan_s* p, int kp, int U);
 void mrhs_free(MrhsTable& t);

@@ -9,6 +9,7 @@
 #include "natural.cuh"
 #include "plan.h"
 #include "solve_kernels.cuh"
+#include "wave4.cuh"
 
 namespace sptrsv {
 
@@ -262,6 +263,7 @@ void plan_free_arrays(sptrsv_plan_s* p)
     layout_free(p->clu);
     strip_free(p->strip);
     wave_free(p->wave);
+    wave4_free(p->wave4);
     cudaFree(p->cptr); cudaFree(p->inv); cudaFree(p->levels); cudaFree(p->lptr); cudaFree(p->ibase); cudaFree(p->ivect);
     for (int j = 0; j < 6; j++) {
         cudaFree(p->ord_tasks[j]);
@@ -333,9 +335,12 @@ int solve_host_streamed(sptrsv_plan_s* p, const double* hb, double* hx_dev, cuda
     double* xbuf = p->hx;
     if (p->part && p->sched.partitions >= 2) {
         lp = p->part->sub;
-        int e = part_ensure(p->part, 1);
-        if (e) return e;
-        xbuf = p->part->xx;
+        xbuf = nullptr;  // the wave4 layout has its own
+        if (!lp->wave4.chunk) {
+            int e = part_ensure(p->part, 1);
+            if (e) return e;
+            xbuf = p->part->xx;
+        }
     }
     lp->launch_bflag = p->bflag;
     lp->launch_seg_rows = seg_rows;
@@ -386,10 +391,11 @@ int plan_fill_values(sptrsv_plan_s* p, const sp_mat_t* L, cudaStream_t s)
         int e = build_cluster_layout(p, H, B);
         if (e) return e;
     }
-    if (p->wave.row) {  // the wave copy
-        const int G = p->wave.G;
+    if (p->wave.row || p->wave4.chunk) {  // the wave copy
+        const int G = p->wave.row ? p->wave.G : p->wave4.G;
         SPT_CUDA(cudaStreamSynchronize(s));
         wave_free(p->wave);
+        wave4_free(p->wave4);
         int e = build_wave_layout(p, G, kWaveMaxRows);
         if (e) return e;
     }
@@ -435,6 +441,40 @@ int plan_ensure_work(sptrsv_plan_s* p, int nrhs)
     return 0;
 }
 
+// A solve over a block system's wave4 layout: b and the results (xo, or x64 per
+// OUT) in the outer plan's rows.
+template <typename V, typename T, typename BT, int OUT, bool STREAM>
+int launch_wave4(sptrsv_plan_s* p, const BT* b, T* xo, double* x64, cudaStream_t s)
+{
+    Ctx* c = ctx();
+    const Wave4Layout& t = p->wave4;
+    const sptrsv_schedule_t& sc = p->sched;
+    const int block = 32 * t.G;
+    const int cap = sc.warps_per_sm > 0 ? (sc.warps_per_sm + t.G - 1) / t.G : 0;
+    T* xp = reinterpret_cast<T*>(t.xp);
+    const V *inv, *lsub, *ev;
+    if constexpr (sizeof(V) == 4) {
+        inv = t.inv32;
+        lsub = t.lsub32;
+        ev = t.ev32;
+    } else {
+        inv = t.inv64;
+        lsub = t.lsub64;
+        ev = t.ev64;
+    }
+    // a streamed solve takes the groups in row order, the order b arrives in
+    const Wave4Mat<V> w{inv, lsub, ev, t.ecol, reinterpret_cast<const int4*>(t.chunk), t.runc, t.grun, t.grow,
+                        STREAM ? nullptr : t.gseq, t.gmap, t.places};
+    auto kern = k_sptrsv_wave4<V, T, BT, OUT, STREAM>;
+    const size_t smem = ((size_t)t.places + 1) * sizeof(T);
+    SPT_CUDA(allow_smem(kern, smem));
+    SPT_CUDA(cudaMemsetAsync(xp, 0xFF, sizeof(T) * (size_t)t.npub, s));
+    SPT_CUDA(launch_persistent_capped(kern, block, smem, t.ngroups, cap, s, w, t.ngroups, b, xp, xo, x64, c->d_status,
+                                      wait_budget_ns(), p->launch_bflag, p->launch_seg_rows, p->launch_epoch,
+                                      p->launch_hx));
+    return 0;
+}
+
 // One sync-free solve over the plan: FP64 (V = T = double) or FP32.
 template <typename V, typename T, typename BT, int OUT>
 int plan_launch(sptrsv_plan_s* p, bool f32, const BT* b, T* x, double* x64, int nrhs, cudaStream_t s)
@@ -469,6 +509,12 @@ int plan_launch(sptrsv_plan_s* p, bool f32, const BT* b, T* x, double* x64, int 
                                                             sc.variant == SPTRSV_VAR_MULTIROW, b, x, x64, s);
         }
     }
+    if (sc.variant == SPTRSV_VAR_WAVE && nrhs == 1) {
+        int e = build_wave_layout(p, sc.block_warps, kWaveMaxRows);
+        if (e) return e;
+        if constexpr (sizeof(V) == 8 && OUT == OUT_X)  // only a streamed host solve comes here with this layout
+            if (p->wave4.chunk) return launch_wave4<V, T, BT, OUT, true>(p, b, nullptr, nullptr, s);
+    }
     // the kernels below wait on x itself: not ready is all ones
     SPT_CUDA(cudaMemsetAsync(x, 0xFF, sizeof(T) * (size_t)n * nrhs, s));
     if (sc.variant == SPTRSV_VAR_CLUSTER && nrhs == 1) {
@@ -502,8 +548,6 @@ int plan_launch(sptrsv_plan_s* p, bool f32, const BT* b, T* x, double* x64, int 
         return 0;
     }
     if (sc.variant == SPTRSV_VAR_WAVE && nrhs == 1) {
-        int e = build_wave_layout(p, sc.block_warps, kWaveMaxRows);
-        if (e) return e;
         const WaveLayout& t = p->wave;
         WaveMat<V> m{{t.row, t.pe, t.ecol,
                       f32 ? reinterpret_cast<const V*>(t.ev32) : reinterpret_cast<const V*>(t.ev64),
@@ -624,6 +668,25 @@ int plan_solve_f64(sptrsv_plan_s* p, const double* b, double* x, int nrhs, cudaS
     return plan_launch<double, double, double, OUT_X>(p, false, b, x, nullptr, nrhs, s);
 }
 
+// A wave4 solve of a block system reads b and writes the results in the outer
+// plan's rows.  Warm-up rows read b of rows that another block writes: where the
+// two overlap, *out = a copy of b.
+template <typename BT, typename X>
+int part_own_rhs(sptrsv_plan_s* p, const BT* b, const X* x, cudaStream_t s, const BT** out)
+{
+    const uintptr_t b0 = (uintptr_t)b, x0 = (uintptr_t)x, m = (uintptr_t)p->n;
+    *out = b;
+    if (!x || x0 >= b0 + m * sizeof(BT) || b0 >= x0 + m * sizeof(X)) return 0;
+    int e = part_ensure(p->part, 1);
+    if (e) return e;
+    BT* copy;
+    if constexpr (sizeof(BT) == 8) copy = p->part->bx;
+    else copy = p->part->bx32;
+    SPT_CUDA(cudaMemcpyAsync(copy, b, sizeof(BT) * (size_t)m, cudaMemcpyDeviceToDevice, s));
+    *out = copy;
+    return 0;
+}
+
 // Partitioned FP64 solve: b gathered into the block system, solved there,
 // each block's real rows scattered into x.
 int part_solve_f64(sptrsv_plan_s* p, const double* b, double* x, int nrhs, cudaStream_t s)
@@ -631,6 +694,11 @@ int part_solve_f64(sptrsv_plan_s* p, const double* b, double* x, int nrhs, cudaS
     PartPlan* q = p->part;
     if (q->sub->sched.variant == SPTRSV_VAR_BAND && nrhs == 1)  // records map to this plan's rows
         return band_solve(q->sub, false, b, false, x, nullptr, OUT_X, s);
+    if (nrhs == 1 && q->sub->sched.variant == SPTRSV_VAR_WAVE && q->sub->wave4.chunk) {
+        int e = part_own_rhs(p, b, x, s, &b);
+        if (e) return e;
+        return launch_wave4<double, double, double, OUT_X, false>(q->sub, b, x, nullptr, s);
+    }
     int e = part_ensure(q, nrhs);
     if (!e) e = part_gather64(q, b, q->bx, nrhs, s);
     if (!e) e = plan_solve_f64(q->sub, q->bx, q->xx, nrhs, s);
@@ -644,6 +712,15 @@ int part_solve32(sptrsv_plan_s* p, const BT* rhs, float* out32, double* x64, int
     PartPlan* q = p->part;
     if (q->sub->sched.variant == SPTRSV_VAR_BAND && nrhs == 1)
         return band_solve(q->sub, true, rhs, sizeof(BT) == 4, out32, x64, out_mode, s);
+    if (nrhs == 1 && q->sub->sched.variant == SPTRSV_VAR_WAVE && q->sub->wave4.chunk) {
+        int e = out_mode == OUT_X ? part_own_rhs(p, rhs, out32, s, &rhs) : part_own_rhs(p, rhs, x64, s, &rhs);
+        if (e) return e;
+        if (out_mode == OUT_SET64)
+            return launch_wave4<float, float, BT, OUT_SET64, false>(q->sub, rhs, nullptr, x64, s);
+        if (out_mode == OUT_ADD64)
+            return launch_wave4<float, float, BT, OUT_ADD64, false>(q->sub, rhs, nullptr, x64, s);
+        return launch_wave4<float, float, BT, OUT_X, false>(q->sub, rhs, out32, nullptr, s);
+    }
     int e = part_ensure(q, nrhs);
     if (e) return e;
     const BT* g;

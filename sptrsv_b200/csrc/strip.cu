@@ -36,6 +36,7 @@
 
 #include "internal.h"
 #include "plan.h"
+#include "wave4.cuh"
 
 namespace sptrsv {
 
@@ -191,7 +192,244 @@ void wave_free(WaveLayout& w)
     w = WaveLayout{};
 }
 
+void wave4_free(Wave4Layout& w)
+{
+    cudaFree(w.inv64); cudaFree(w.inv32); cudaFree(w.lsub64); cudaFree(w.lsub32); cudaFree(w.ev64); cudaFree(w.ev32);
+    cudaFree(w.ecol); cudaFree(w.chunk); cudaFree(w.runc); cudaFree(w.grun); cudaFree(w.grow); cudaFree(w.gseq);
+    cudaFree(w.gmap); cudaFree(w.xp);
+    w = Wave4Layout{};
+}
+
+bool wave_built(const sptrsv_plan_s* p, int G)
+{
+    return (p->wave.row && p->wave.G == G) || (p->wave4.chunk && p->wave4.G == G);
+}
+
 namespace {
+
+// bad |= 1 where a row has more than one entry beside the one on the row before,
+// or that one lies inside the row's chunk, or the row before counts for more
+// than the row itself (a scan over 128 rows multiplies these factors: they must
+// not grow).  pub[q] = 1 for chunks that another group reads.
+__global__ void k_wave4_check(SptLayout l, const int* __restrict__ inv, int n, const int* __restrict__ rchunk,
+                              const int* __restrict__ cstart, const int* __restrict__ cgroup, int* pub, int* bad)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int q = rchunk[i], p = inv[i];
+        int cnt = 0;
+        bool no = false;
+        for (int t = l.ptr[p]; t < l.ptr[p + 1]; t++) {
+            const int c = l.col[t];
+            if (c == i - 1) {
+                no |= !(fabs(l.val64[t] * l.di64[p]) <= 1.0);
+                continue;
+            }
+            no |= ++cnt > 1 || c >= cstart[q];
+            if (cgroup[rchunk[c]] != cgroup[q]) pub[rchunk[c]] = 1;
+        }
+        if (no) *bad = 1;
+    }
+}
+
+// Every slot, the ones without a row included (place `zero`: a constant 0).
+__global__ void k_wave4_fill(SptLayout l, const int* __restrict__ inv, int nch, const int* __restrict__ rchunk,
+                             const int* __restrict__ cgroup, int zero, const int4* __restrict__ chunk,
+                             double* __restrict__ inv64, float* __restrict__ inv32, double* __restrict__ lsub64,
+                             float* __restrict__ lsub32, double* __restrict__ ev64, float* __restrict__ ev32,
+                             int* __restrict__ ecol)
+{
+    constexpr int Q = kWave4Q, C = kWave4C;
+    for (long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x; s < (long long)nch * C;
+         s += (long long)gridDim.x * blockDim.x) {
+        const int q = (int)(s / C), o = (int)(s % C);
+        const int4 m = chunk[q];
+        const int r = m.x + o;
+        double di = 0, ls = 0, ev = 0;
+        float di32 = 0;
+        int ec = ~zero;
+        if (o < m.y) {
+            const int p = inv[r];
+            di = l.di64[p];
+            di32 = l.di32[p];
+            for (int t = l.ptr[p]; t < l.ptr[p + 1]; t++) {
+                const int c = l.col[t];
+                if (c == r - 1) {
+                    ls = l.val64[t];
+                    continue;
+                }
+                const int qc = rchunk[c];
+                const int4 mc = chunk[qc];
+                const int pc = c - mc.x, lanes = (mc.y + Q - 1) / Q;
+                ec = cgroup[qc] == cgroup[q] ? ~(mc.z + pc % Q * lanes + pc / Q) : mc.w + pc;
+                ev = l.val64[t];
+            }
+        }
+        inv64[s] = di;
+        inv32[s] = di32;
+        lsub64[s] = ls;
+        lsub32[s] = (float)ls;
+        ev64[s] = ev;
+        ev32[s] = (float)ev;
+        ecol[s] = ec;
+    }
+}
+
+// Groups of G consecutive lines (fewer at a block's end), by the first rows of
+// the lines.  seq: the processing order, empty for the natural one; on a block
+// system the blocks' groups interleaved (the j-th of every block, then the
+// (j+1)-th), which is topological because a group depends only on groups of its
+// own block.
+struct WaveGroups {
+    std::vector<int> grun, seq, blk;
+    void make(const sptrsv_plan_s* p, const std::vector<int>& run_row, int G)
+    {
+        const int nruns = (int)run_row.size();
+        size_t nb = 0;  // blocks whose start is at or before the current run
+        int in_group = 0;
+        for (int r = 0; r < nruns; r++) {
+            bool starts_block = false;
+            while (nb < p->blk_starts.size() && p->blk_starts[nb] <= run_row[r]) {
+                starts_block = p->blk_starts[nb] == run_row[r];
+                nb++;
+            }
+            if (r == 0 || in_group == G || starts_block) {
+                grun.push_back(r);
+                blk.push_back(nb > 0 ? (int)nb - 1 : 0);
+                in_group = 0;
+            }
+            in_group++;
+        }
+        grun.push_back(nruns);
+        const int ng = (int)blk.size();
+        if (p->blk_starts.empty() || ng == 0) return;
+        std::vector<int> rank(ng);
+        for (int g = 0; g < ng; g++) rank[g] = (g > 0 && blk[g] == blk[g - 1]) ? rank[g - 1] + 1 : 0;
+        seq.resize(ng);
+        for (int g = 0; g < ng; g++) seq[g] = g;
+        std::stable_sort(seq.begin(), seq.end(), [&](int a, int b) { return rank[a] < rank[b]; });
+    }
+};
+
+// The layout of wave4.cuh; SPTRSV_ERR_UNSUPPORTED (no message) when the block
+// system does not have its form.
+int build_wave4(sptrsv_plan_s* p, int G, int max_rows)
+{
+    constexpr int Q = kWave4Q, C = kWave4C;
+    const int n = p->n;
+    cudaStream_t s = 0;
+    Wave4Layout w{};
+    unsigned char* brk = nullptr;
+    int *rch = nullptr, *cst = nullptr, *cgr = nullptr, *res = nullptr;  // res: pub per chunk, then bad
+    auto cleanup = [&]() {
+        cudaFree(brk); cudaFree(rch); cudaFree(cst); cudaFree(cgr); cudaFree(res);
+    };
+    auto fail = [&](int code) {
+        cleanup();
+        wave4_free(w);
+        return code;
+    };
+#define W4CHK(call)                                               \
+    do {                                                          \
+        cudaError_t e_ = (call);                                  \
+        if (e_ != cudaSuccess) return fail(cuda_fail(e_, #call)); \
+    } while (0)
+    W4CHK(dalloc(&brk, n));
+    k_strip_breaks<<<grid_for(n, 256), 256, 0, s>>>(p->lev, p->inv, n, brk);
+    W4CHK(cudaGetLastError());
+    std::vector<unsigned char> hbrk(n);
+    W4CHK(cudaMemcpy(hbrk.data(), brk, (size_t)n, cudaMemcpyDeviceToHost));
+    // chunks and runs
+    std::vector<int> cstart, rchunk(n), run0, run_row;
+    for (int i = 0; i < n; i++) {
+        if (hbrk[i]) {
+            run0.push_back((int)cstart.size());
+            run_row.push_back(i);
+        }
+        if (hbrk[i] || i - cstart.back() == C) cstart.push_back(i);
+        rchunk[i] = (int)cstart.size() - 1;
+    }
+    const int nch = (int)cstart.size(), nruns = (int)run0.size();
+    cstart.push_back(n);
+    run0.push_back(nch);
+    WaveGroups gr;
+    gr.make(p, run_row, G);
+    const int ng = (int)gr.blk.size();
+    std::vector<int> grow(ng + 1), cgroup(nch), hchunk(4 * (size_t)nch, 0);
+    int places = 0;
+    for (int g = 0; g < ng; g++) {
+        grow[g] = run_row[gr.grun[g]];
+        int at = 0;
+        for (int q = run0[gr.grun[g]]; q < run0[gr.grun[g + 1]]; q++) {
+            const int rows = cstart[q + 1] - cstart[q];
+            cgroup[q] = g;
+            hchunk[4 * (size_t)q] = cstart[q];
+            hchunk[4 * (size_t)q + 1] = rows;
+            hchunk[4 * (size_t)q + 2] = at;
+            at += (rows + Q - 1) / Q * Q;
+        }
+        places = std::max(places, at);
+    }
+    grow[ng] = n;
+    if (places + 1 > max_rows) return fail(SPTRSV_ERR_UNSUPPORTED);
+    W4CHK(dalloc(&rch, n));
+    W4CHK(dalloc(&cst, nch + 1));
+    W4CHK(dalloc(&cgr, nch));
+    W4CHK(dalloc(&res, nch + 1));
+    W4CHK(cudaMemcpy(rch, rchunk.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
+    W4CHK(cudaMemcpy(cst, cstart.data(), sizeof(int) * ((size_t)nch + 1), cudaMemcpyHostToDevice));
+    W4CHK(cudaMemcpy(cgr, cgroup.data(), sizeof(int) * (size_t)nch, cudaMemcpyHostToDevice));
+    W4CHK(cudaMemsetAsync(res, 0, sizeof(int) * ((size_t)nch + 1), s));
+    k_wave4_check<<<grid_for(n, 256), 256, 0, s>>>(p->lev, p->inv, n, rch, cst, cgr, res, res + nch);
+    W4CHK(cudaGetLastError());
+    std::vector<int> pub(nch + 1);
+    W4CHK(cudaMemcpy(pub.data(), res, sizeof(int) * pub.size(), cudaMemcpyDeviceToHost));
+    if (pub[nch]) return fail(SPTRSV_ERR_UNSUPPORTED);
+    for (int q = 0; q < nch; q++) {
+        hchunk[4 * (size_t)q + 3] = pub[q] ? w.npub : -1;
+        if (pub[q]) w.npub += (hchunk[4 * (size_t)q + 1] + Q - 1) / Q * Q;
+    }
+    W4CHK(dalloc(&w.xp, std::max(1, w.npub)));
+    const long long ns = (long long)nch * C;
+    W4CHK(dalloc(&w.inv64, ns));
+    W4CHK(dalloc(&w.inv32, ns));
+    W4CHK(dalloc(&w.lsub64, ns));
+    W4CHK(dalloc(&w.lsub32, ns));
+    W4CHK(dalloc(&w.ev64, ns));
+    W4CHK(dalloc(&w.ev32, ns));
+    W4CHK(dalloc(&w.ecol, ns));
+    W4CHK(dalloc(&w.chunk, 4LL * nch));
+    W4CHK(dalloc(&w.runc, nruns + 1));
+    W4CHK(dalloc(&w.grun, ng + 1));
+    W4CHK(dalloc(&w.grow, ng + 1));
+    W4CHK(cudaMemcpy(w.chunk, hchunk.data(), sizeof(int) * hchunk.size(), cudaMemcpyHostToDevice));
+    W4CHK(cudaMemcpy(w.runc, run0.data(), sizeof(int) * (size_t)(nruns + 1), cudaMemcpyHostToDevice));
+    W4CHK(cudaMemcpy(w.grun, gr.grun.data(), sizeof(int) * (size_t)(ng + 1), cudaMemcpyHostToDevice));
+    W4CHK(cudaMemcpy(w.grow, grow.data(), sizeof(int) * (size_t)(ng + 1), cudaMemcpyHostToDevice));
+    if (!gr.seq.empty()) {
+        W4CHK(dalloc(&w.gseq, ng));
+        W4CHK(cudaMemcpy(w.gseq, gr.seq.data(), sizeof(int) * (size_t)ng, cudaMemcpyHostToDevice));
+    }
+    std::vector<int> gm(2 * (size_t)ng);  // a group's rows in the outer plan
+    for (int g = 0; g < ng; g++) {
+        const int* t = &p->part_tab[4 * (size_t)gr.blk[g]];  // s, a, e, base
+        gm[2 * (size_t)g] = t[0] + (grow[g] - t[3]);
+        gm[2 * (size_t)g + 1] = std::max(0, std::min(grow[g + 1] - grow[g], t[3] + (t[1] - t[0]) - grow[g]));
+    }
+    W4CHK(dalloc(&w.gmap, 2LL * ng));
+    W4CHK(cudaMemcpy(w.gmap, gm.data(), sizeof(int) * gm.size(), cudaMemcpyHostToDevice));
+    k_wave4_fill<<<grid_for(ns, 256), 256, 0, s>>>(p->lev, p->inv, nch, rch, cgr, places,
+                                                  reinterpret_cast<const int4*>(w.chunk), w.inv64, w.inv32, w.lsub64, w.lsub32,
+                                                  w.ev64, w.ev32, w.ecol);
+    W4CHK(cudaGetLastError());
+    W4CHK(cudaStreamSynchronize(s));
+#undef W4CHK
+    w.ngroups = ng;
+    w.G = G;
+    w.places = places;
+    cleanup();
+    p->wave4 = w;
+    return 0;
+}
 
 // The chunk cut and the per-row data both layouts start from.
 struct Chunks {
@@ -416,8 +654,13 @@ int build_strip_layout(sptrsv_plan_s* p, int R)
 
 int build_wave_layout(sptrsv_plan_s* p, int G, int max_rows)
 {
-    if (p->wave.row && p->wave.G == G) return 0;
+    if (wave_built(p, G)) return 0;
     wave_free(p->wave);
+    wave4_free(p->wave4);
+    if (!p->part_tab.empty()) {  // block systems of 2D stencils: four rows a lane; else a row a lane
+        const int e = build_wave4(p, G, max_rows);
+        if (e != SPTRSV_ERR_UNSUPPORTED) return e;
+    }
     cudaStream_t s = 0;
     WaveLayout w{};
     Chunks ch;
@@ -448,44 +691,17 @@ int build_wave_layout(sptrsv_plan_s* p, int G, int max_rows)
         if (q == 0 || !ch.linked[q]) run0.push_back(q);
     const int nruns = (int)run0.size();
     run0.push_back(nch);
-    std::vector<int> grun, blk_of_group;
-    {
-        size_t nb = 0;  // blocks whose start is at or before the current run
-        int in_group = 0;
-        for (int r = 0; r < nruns; r++) {
-            const int row = ch.cstart[run0[r]];
-            bool starts_block = false;
-            while (nb < p->blk_starts.size() && p->blk_starts[nb] <= row) {
-                starts_block = p->blk_starts[nb] == row;
-                nb++;
-            }
-            if (r == 0 || in_group == G || starts_block) {
-                grun.push_back(r);
-                blk_of_group.push_back(nb > 0 ? (int)nb - 1 : 0);
-                in_group = 0;
-            }
-            in_group++;
-        }
-        grun.push_back(nruns);
-    }
+    std::vector<int> run_row(nruns);
+    for (int r = 0; r < nruns; r++) run_row[r] = ch.cstart[run0[r]];
+    WaveGroups gr;
+    gr.make(p, run_row, G);
+    const std::vector<int>&grun = gr.grun, &gseq = gr.seq;
     const int ngroups = (int)grun.size() - 1;
     std::vector<int> grow(ngroups + 1), g0(nch), ident(nch);
     int cap = 0;
     for (int g = 0; g <= ngroups; g++) {
         grow[g] = ch.cstart[run0[grun[g]]];
         if (g > 0) cap = std::max(cap, grow[g] - grow[g - 1]);
-    }
-    // processing order: natural, or on a block system the blocks' groups
-    // interleaved (the j-th group of every block, then the (j+1)-th), which is
-    // topological because a group depends only on groups of its own block
-    std::vector<int> gseq;
-    if (!p->blk_starts.empty() && ngroups > 0) {
-        std::vector<int> rank(ngroups);
-        for (int g = 0; g < ngroups; g++)
-            rank[g] = (g > 0 && blk_of_group[g] == blk_of_group[g - 1]) ? rank[g - 1] + 1 : 0;
-        gseq.resize(ngroups);
-        for (int g = 0; g < ngroups; g++) gseq[g] = g;
-        std::stable_sort(gseq.begin(), gseq.end(), [&](int a, int b) { return rank[a] < rank[b]; });
     }
     if (cap > max_rows)
         return fail(set_error(SPTRSV_ERR_UNSUPPORTED, "wave schedule: %d lines of the matrix hold %d rows, more than "
