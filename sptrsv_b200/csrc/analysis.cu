@@ -312,6 +312,50 @@ __global__ void k_keys(const int* __restrict__ rowptr, const int* __restrict__ l
     }
 }
 
+// Is the matrix a stencil on lines of equal length (lines.cuh)?  stats[16] = the
+// length w, 0: no; from the distance of 32 sampled rows to their last column
+// that is not the row before.
+__global__ void k_line_width(const int* __restrict__ rowptr, const int* __restrict__ col, int n, int* stats)
+{
+    const int r = (int)((long long)n * (threadIdx.x + 1) / 33);
+    int z = rowptr[r + 1] - 2, d = 0;
+    if (z >= rowptr[r] && col[z] == r - 1) z--;
+    if (z >= rowptr[r]) d = r - col[z];
+    const unsigned same = __match_any_sync(0xffffffffu, d);
+    const int votes = d ? __popc(same) : 0;
+    const int most = __reduce_max_sync(0xffffffffu, votes);
+    const unsigned who = __ballot_sync(0xffffffffu, votes == most);
+    if (threadIdx.x == __ffs(who) - 1) stats[16] = most >= 16 ? d : 0;
+}
+
+// stats[17] |= 1 where a row has more than kLineOff off-diagonals, or one inside
+// its chunk of 32 (cut at line starts) beside the row before; stats[18] = the most
+// of a row; stats[19] = lines whose first row reads the row before.
+__global__ void k_line_check(const int* __restrict__ rowptr, const int* __restrict__ col, int n, int* stats)
+{
+    const int w = stats[16];
+    int most = 0, joined = 0;
+    bool bad = w < 32;
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n && !bad; r += gridDim.x * blockDim.x) {
+        const int p = r % w, c0 = r - p % 32, s = rowptr[r], e = rowptr[r + 1] - 1;
+        most = max(most, e - s);
+        bad = e - s > kLineOff;
+        for (int z = s; z < e && !bad; z++) {
+            const int c = col[z];
+            if (c == r - 1) joined += p == 0;
+            else bad = c >= c0;
+        }
+    }
+    bad = __any_sync(0xffffffffu, bad);
+    most = __reduce_max_sync(0xffffffffu, most);
+    joined = __reduce_add_sync(0xffffffffu, joined);
+    if ((threadIdx.x & 31) == 0) {
+        if (bad) stats[17] = 1;
+        if (most) atomicMax(stats + 18, most);
+        if (joined) atomicAdd(stats + 19, joined);
+    }
+}
+
 // warps per key (get_warps_per_bucks :66-71 with get_size_from_pos :84-102)
 __global__ void k_warps_per_key(const int* __restrict__ counts, int K, int* __restrict__ wpk)
 {
@@ -489,9 +533,13 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     rec->d_lptr = d_levsz + part((long long)nlevs + 1);
     int* d_stats = rec->d_lptr + part((long long)nlevs + 1);
     ACHK(cudaMemsetAsync(rec->d_counts, 0, sizeof(int) * (size_t)(K + 1), s));
-    ACHK(cudaMemsetAsync(d_stats, 0, 16 * sizeof(int), s));
+    ACHK(cudaMemsetAsync(d_stats, 0, sizeof(rec->stats), s));
     if (n > 0) {
         k_keys<<<grid_for(n, 256), 256, 0, s>>>(L->ia, rec->d_levels, n, d_key, d_iorder, rec->d_counts, d_stats + 15);
+        ACHK(cudaGetLastError());
+        k_line_width<<<1, 32, 0, s>>>(L->ia, L->ja, n, d_stats);
+        ACHK(cudaGetLastError());
+        k_line_check<<<grid_for(n, 256), 256, 0, s>>>(L->ia, L->ja, n, d_stats);
         ACHK(cudaGetLastError());
         ACHK(radix_sort_pairs(d_key, d_iorder, d_key2, d_val2, n, (int)(K - 1), d_scr, s));
     }
@@ -514,7 +562,7 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
         k_level_sizes<<<grid_for(nlevs + 1LL, 256), 256, 0, s>>>(rec->d_counts, d_rowoff, nlevs, d_levsz, rec->d_lptr,
                                                                  d_stats);
         ACHK(cudaGetLastError());
-        ACHK(cudaMemcpyAsync(rec->stats, d_stats, 16 * sizeof(int), cudaMemcpyDeviceToHost, s));
+        ACHK(cudaMemcpyAsync(rec->stats, d_stats, sizeof(rec->stats), cudaMemcpyDeviceToHost, s));
         ACHK(cudaMemcpyAsync(&n_warps, d_wpk + K, sizeof(int), cudaMemcpyDeviceToHost, s));
         ACHK(cudaStreamSynchronize(s));
     }

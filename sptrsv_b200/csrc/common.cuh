@@ -98,6 +98,9 @@ __device__ __forceinline__ float publishable(float v)
     return __float_as_uint(v) == 0xFFFFFFFFu ? __uint_as_float(0x7FC00000u) : v;
 }
 
+__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7FF00000) != 0x7FF00000; }
+__device__ __forceinline__ bool finite_bits(float v) { return (__float_as_int(v) & 0x7F800000) != 0x7F800000; }
+
 __device__ __forceinline__ void report(DevStatus* st, int code, int row)
 {
     if (atomicCAS(&st->code, 0, code) == 0) st->row = row;

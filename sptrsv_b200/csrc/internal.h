@@ -184,7 +184,7 @@ struct AnalysisRec {
     int* d_ivect = nullptr;    // [n_warps]
     int* d_wlev = nullptr;     // [n_warps]
     int* d_lptr = nullptr;     // [nlevs+1] first iorder position of each level
-    int stats[16] = {};        // level widths and row lengths (k_level_sizes)
+    int stats[20] = {};        // level widths and row lengths (k_level_sizes), grid lines (k_line_check)
     int* slab[3] = {};         // the allocations that hold these arrays and the info struct's
     bool map_in_info = false;  // map arrays are also referenced by the info struct
     int* tile_tasks[6] = {};   // level-aligned iorder tasks for 32>>j lanes per row
@@ -195,7 +195,8 @@ struct AnalysisRec {
 struct LevelCtaShape {
     int kp, g;
 };
-LevelCtaShape choose_level_cta(int nlevs, int n, const int* stats, bool level_ordered);
+LevelCtaShape choose_level_cta(int nlevs, int n, const int* stats, bool level_ordered, double* cycles);
+constexpr int kLineOff = 5;  // most off-diagonals of a row in lines.cuh
 void register_analysis(const int* key, AnalysisRec* rec);
 
 // Rows of one task of the level kernel (one CTA, one thread per row).

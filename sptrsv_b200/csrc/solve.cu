@@ -6,6 +6,7 @@
 
 #include "internal.h"
 #include "level_cta.cuh"
+#include "lines.cuh"
 #include "natural.cuh"
 #include "plan.h"
 #include "solve_kernels.cuh"
@@ -58,6 +59,45 @@ __global__ void k_iorder_level_keys(const int* __restrict__ iorder, const int* _
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) key[p] = level[iorder[p]] - 1;
 }
 
+// Lines of w rows, G a CTA, up to U off-diagonals a row; w = 0: not by lines.
+struct LineShape {
+    int w, G, U;
+};
+
+// By lines where that is estimated to take fewer cycles than the levels do.  A
+// line behind the one above costs 710 cycles (100 x 3000 grid: 0.37 us; in 3D,
+// where more of them are hops between CTAs, 1,400 for 101 x 90 x 97), a chunk
+// along the line 2,300 (3000 x 100: 1.2 us), the start 10,000.  On wide levels
+// one CTA takes 0.62 of its estimate (100 x 1000: 341 us, by lines 371; 200 x
+// 200: 197 and 88; 61 x 47: 18 and 28), the sync-free kernels always more than
+// by lines from 32 rows a line on.
+LineShape choose_lines(int nlevs, int n, const int* stats, double levels)
+{
+    const int w = stats[16], U = stats[18] <= 2 ? 2 : stats[18] == 3 ? 3 : kLineOff;
+    LineShape sh{0, 0, U};
+    if (w < 32 || stats[17]) return sh;
+    const int nlines = div_up(n, w);
+    if (710.0 * std::max(nlevs - w, 0) + 2300.0 * div_up(w, 32) + 10000 > levels) return sh;
+    if (10LL * stats[19] > nlines) return sh;  // not where the lines start
+    const size_t stage = 2 * line_stage_bytes(U);
+    for (int G = kLineG; G >= 2 && !sh.G; G /= 2)
+        if (G * (sizeof(double) * w + stage) <= 200 * 1024 && (long long)G * w + n < 0x7fffff00) sh.G = G;
+    if (!sh.G) return sh;
+    sh.w = w;
+    return sh;
+}
+
+template <int U>
+int launch_lines(const sp_mat_t* mat, LineShape sh, const double* b, double* x, int n, cudaStream_t s)
+{
+    const size_t smem = sh.G * (sizeof(double) * sh.w + 2 * line_stage_bytes(U));
+    auto kern = k_sptrsv_lines<U>;
+    SPT_CUDA(allow_smem(kern, smem));
+    SPT_CUDA(launch_persistent(kern, 32 * sh.G, smem, div_up(n, sh.G * sh.w), s, mat->ia, mat->ja, mat->a, n, sh.w, sh.G, b,
+                               x, ctx()->d_status, wait_budget_ns()));
+    return 0;
+}
+
 // Level-aligned tasks over iorder for `lanes` lanes per row, cached with the analysis.
 int tile_tasks(AnalysisRec* rec, const int* iorder, int lanes, const int** tasks, int* ntasks)
 {
@@ -90,7 +130,7 @@ int tile_tasks(AnalysisRec* rec, const int* iorder, int lanes, const int** tasks
 // level with a row of more than 4 kp entries, 2,600 more.  The sync-free
 // kernels: 1,600 to 1,900 a level whatever its width up to some thousand rows
 // (832, 4095 and 6219 levels).
-LevelCtaShape choose_level_cta(int nlevs, int n, const int* stats, bool level_ordered)
+LevelCtaShape choose_level_cta(int nlevs, int n, const int* stats, bool level_ordered, double* cycles)
 {
     static const double kBase[4] = {260, 330, 430, 850};
     const double extra = 2600, rows = (level_ordered ? 8.0 : 11.0) * n;
@@ -109,6 +149,7 @@ LevelCtaShape choose_level_cta(int nlevs, int n, const int* stats, bool level_or
             }
         }
     }
+    if (cycles) *cycles = best_cost;
     return best;
 }
 
@@ -156,10 +197,18 @@ int solve_reference(sp_mat_t* mat, dfr_analysis_info_t* info, const double* b, d
     if (mode != SIMPLE && (!info || !info->iorder))
         return set_error(SPTRSV_ERR_NOT_ANALYSED, "solve: ORDER/MULTIROW need an analysis");
     if (lanes && !pow2_lanes(lanes)) return set_error(SPTRSV_ERR_INVALID_ARG, "solve: lanes must be 1,2,4,8,16,32");
-    if (mode != SIMPLE) {
-        // few rows per level: one CTA (its result does not depend on `lanes`)
-        AnalysisRec* rec = find_analysis(info->row_ctr);
-        const LevelCtaShape sh = rec && rec->n == n ? choose_level_cta(rec->nlevs, n, rec->stats, false) : LevelCtaShape{0, 0};
+    AnalysisRec* rec = mode != SIMPLE ? find_analysis(info->row_ctr) : nullptr;
+    if (rec && rec->n == n) {
+        // few rows per level: one CTA; stencils: by lines (the results do not depend on `lanes`)
+        double cycles;
+        const LevelCtaShape sh = choose_level_cta(rec->nlevs, n, rec->stats, false, &cycles);
+        const LineShape ln = choose_lines(rec->nlevs, n, rec->stats, sh.kp ? 0.62 * cycles : cycles);
+        if (ln.w) {
+            SPT_CUDA(cudaMemsetAsync(x, 0xFF, sizeof(double) * (size_t)n, s));
+            int e = ln.U == 2 ? launch_lines<2>(mat, ln, b, x, n, s)
+                    : ln.U == 3 ? launch_lines<3>(mat, ln, b, x, n, s) : launch_lines<kLineOff>(mat, ln, b, x, n, s);
+            return e ? e : ok();
+        }
         if (sh.kp) {
             const NatMat m{mat->ia, mat->ja, mat->a, info->iorder, mat->nnz};
             int e = launch_level_cta<NatMat, double, double, OUT_X>(m, sh, rec->d_lptr, info->inv_iorder, rec->nlevs, n,
@@ -176,7 +225,6 @@ int solve_reference(sp_mat_t* mat, dfr_analysis_info_t* info, const double* b, d
         const int* ivect = info->ivect_size_warp;
         int nw = info->n_warps;
         if (!ibase) {  // analysed in ORDER mode: use the map kept with the analysis
-            AnalysisRec* rec = find_analysis(info->row_ctr);
             if (!rec) return set_error(SPTRSV_ERR_NOT_ANALYSED, "solve: no multirow map for this analysis");
             ibase = rec->d_ibase;
             ivect = rec->d_ivect;
@@ -187,7 +235,6 @@ int solve_reference(sp_mat_t* mat, dfr_analysis_info_t* info, const double* b, d
     } else if (mode == ORDER && lanes && lanes < 32) {
         // order with a tile of `lanes` lanes: tasks never cross a level, so the
         // rows of one warp are independent
-        AnalysisRec* rec = find_analysis(info->row_ctr);
         if (!rec) return set_error(SPTRSV_ERR_NOT_ANALYSED, "solve: no analysis record for this info");
         const int* tasks = nullptr;
         int ntasks = 0;
@@ -500,7 +547,7 @@ int plan_launch(sptrsv_plan_s* p, bool f32, const BT* b, T* x, double* x64, int 
     if (sc.variant == SPTRSV_VAR_BAND && nrhs == 1)
         return band_solve(p, f32, b, sizeof(BT) == 4, x, x64, OUT, s);
     if ((sc.variant == SPTRSV_VAR_ORDER || sc.variant == SPTRSV_VAR_MULTIROW) && nrhs == 1) {
-        const LevelCtaShape sh = choose_level_cta(p->nlevs, n, p->stats, true);
+        const LevelCtaShape sh = choose_level_cta(p->nlevs, n, p->stats, true, nullptr);
         if (sh.kp) {
             const V *val, *dg, *di;
             layout_vals(p->lev, val, dg, di);

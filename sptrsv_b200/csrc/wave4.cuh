@@ -98,9 +98,6 @@ __device__ __forceinline__ void ldg_vec(const E* p, E (&r)[N])
     }
 }
 
-__device__ __forceinline__ bool finite_bits(double v) { return (__double2hiint(v) & 0x7FF00000) != 0x7FF00000; }
-__device__ __forceinline__ bool finite_bits(float v) { return (__float_as_int(v) & 0x7F800000) != 0x7F800000; }
-
 __device__ __forceinline__ void st_relaxed2(double* p, double a, double b)
 {
     asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(a), "d"(b) : "memory");
