@@ -739,9 +739,13 @@ __global__ void __launch_bounds__(512, 1) k_sptrsv_strip(StripMat<V> m, int nstr
 // grid), else U = kStripU.  MULTI: some row holds more than U such entries
 // (later rounds load theirs on the spot); STREAM: the streamed host solve.
 //
-// The scan's products of beta are formed before the wait, and x goes to shared
-// memory before anything of the next chunk (2048 x 2048, 8 lines a CTA: 884 ->
-// 819 us; 333 x 277: 121 -> 114 us; 101 x 90 x 97: 188 -> 179 us).
+// Bound by the lag from a line to the next, so what does not hang on the line
+// above comes before the wait: the scan's products of beta, the x64 that a
+// refinement adds to, and (rows of up to U entries) a first look at x of other
+// groups, in 3D long known when the line above in the group is not.  x goes to
+// shared memory before anything of the next chunk.  8 lines a CTA, FP64:
+// 2048 x 2048 884 -> 766 us, 333 x 277 121 -> 107 us, 101 x 90 x 97 188 -> 154 us
+// (refined 466 -> 420 us).
 template <typename V>
 struct WaveMat {
     StripMat<V> c;                 // slot arrays (sptr unused)
@@ -808,6 +812,22 @@ __global__ void __launch_bounds__(512, 1) k_sptrsv_wave(WaveMat<V> w, int ngroup
                     strip_ent<V, T, BT, U>(e0, m0, m, b, STREAM);
                     if (q + 2 < q1) strip_meta<V, T>(m1, m, (q + 2) * 32 + lane);
                 }
+                const int ec = md.e1 - md.e0;
+                // x of other groups, mostly long known: under way first
+                bool glob = false;
+                T xv0[U];
+                double old = 0;  // OUT_ADD64
+                if (OUT == OUT_ADD64 && md.row >= 0) old = x64[md.row];
+                if (!MULTI) {
+#pragma unroll
+                    for (int u = 0; u < U; u++) glob |= u < ec && en.cc[u] >= 0;
+                    glob = __any_sync(FULL, glob);
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        xv0[u] = (T)0;
+                        if (glob && u < ec && en.cc[u] >= 0) xv0[u] = ld_relaxed(x + en.cc[u]);
+                    }
+                }
                 // the scan's products of beta over 2^d lanes, before the wait
                 T M[5], bb = -md.lsub * md.piv;
 #pragma unroll
@@ -816,9 +836,41 @@ __global__ void __launch_bounds__(512, 1) k_sptrsv_wave(WaveMat<V> w, int ngroup
                     const T bp = __shfl_up_sync(FULL, bb, 1 << d);
                     if (lane >= (1 << d)) bb *= bp;
                 }
-                const int ec = md.e1 - md.e0;
                 T acc = en.b;
-                const int rounds = MULTI ? __reduce_max_sync(FULL, ec) : 1;
+                if (!MULTI) {
+                    unsigned it = 0;
+                    unsigned long long t0 = 0;
+                    while (glob) {
+                        bool pend = false;
+#pragma unroll
+                        for (int u = 0; u < U; u++) pend |= is_pending(xv0[u]);
+                        if (!__any_sync(FULL, pend)) break;
+                        if ((++it & 63u) == 0 && give_up(t0, st, budget, md.row)) {
+                            failed = true;
+                            break;
+                        }
+                        if (backoff && it > 4) __nanosleep(backoff);
+#pragma unroll
+                        for (int u = 0; u < U; u++)
+                            if (u < ec && en.cc[u] >= 0) xv0[u] = ld_relaxed(x + en.cc[u]);
+                    }
+                    while (!failed) {
+                        bool pend = false;
+#pragma unroll
+                        for (int u = 0; u < U; u++)
+                            if (u < ec && en.cc[u] < 0) xv0[u] = xs[~en.cc[u]];
+#pragma unroll
+                        for (int u = 0; u < U; u++) pend |= is_pending(xv0[u]);
+                        if (!__any_sync(FULL, pend)) break;
+                        if ((++it & 63u) == 0 && give_up(t0, st, budget, md.row)) failed = true;
+                        if (backoff && it > 4) __nanosleep(backoff);
+                    }
+                    if (failed) break;
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (u < ec) acc -= en.vv[u] * xv0[u];
+                }
+                const int rounds = MULTI ? __reduce_max_sync(FULL, ec) : 0;
                 for (int j = 0; j < rounds; j += U) {
                     const int nh = min(U, ec - j);
                     int cc[U];
@@ -827,7 +879,7 @@ __global__ void __launch_bounds__(512, 1) k_sptrsv_wave(WaveMat<V> w, int ngroup
                     for (int u = 0; u < U; u++) {
                         cc[u] = en.cc[u];
                         vv[u] = en.vv[u];
-                        if (MULTI && j > 0) {
+                        if (j > 0) {
                             cc[u] = 0;
                             vv[u] = 0;
                             if (u < nh) {
@@ -854,7 +906,11 @@ __global__ void __launch_bounds__(512, 1) k_sptrsv_wave(WaveMat<V> w, int ngroup
                 const T xi = publishable(a);
                 if (md.row >= 0) xs[md.row - r0] = xi;
                 __syncwarp();  // nothing of what follows ahead of the store that the line below waits for
-                if (md.row >= 0) publish<T, OUT>(x, x64, md.row, xi);
+                if (md.row >= 0) {
+                    st_relaxed(x + md.row, xi);
+                    if (OUT == OUT_SET64) x64[md.row] = (double)xi;
+                    if (OUT == OUT_ADD64) x64[md.row] = old + (double)xi;
+                }
             }
         }
         if (failed && lane == 0) abort_flag = 1;

@@ -24,8 +24,8 @@
 //   1000 x 900,  16 blocks  106 / 350 ->  67 / 216
 //   333 x 277,   16 blocks   53 / 156 ->  41 / 116
 // An unpartitioned system is one chain of hops from group to group, where a hop
-// costs this kernel more (2048 x 2048, 4 lines a CTA: 892 against 997 us;
-// 101 x 90 x 97, two couplings: 159 against 225 us): it keeps the other form.
+// costs this kernel more (2048 x 2048, 4 lines a CTA: 856 against 997 us;
+// 101 x 90 x 97, two couplings: 144 against 225 us): it keeps the other form.
 //
 // What keeps the lag short is the order of instructions: a chunk's x is stored
 // before anything of the next chunk is loaded, held there by __syncwarp() (left
