@@ -642,7 +642,10 @@ int plan_launch(sptrsv_plan_s* p, bool f32, const BT* b, T* x, double* x64, int 
         if (t.nsplit) SPT_CUDA(cudaMemsetAsync(t.pcnt, 0, sizeof(int) * (size_t)t.nsplit, s));
         // rows of x a whole number of 16-byte copies wide: gathered through L2 in 16-byte copies
         const bool cg = (nrhs * sizeof(T)) % 16 == 0;
-        auto kern = U == 8 ? (cg ? k_sptrsv_mrhs<V, T, BT, OUT, 8, MRHS_CG> : k_sptrsv_mrhs<V, T, BT, OUT, 8, MRHS_CA>)
+        // long rows on wide levels (k_sptrsv_mrhs): a row's lanes share its entries out
+        const bool spread = cg && U == 16 && kp >= U && p->nnz_off >= 8LL * n;
+        auto kern = spread ? k_sptrsv_mrhs<V, T, BT, OUT, 16, MRHS_CG, true>
+                    : U == 8 ? (cg ? k_sptrsv_mrhs<V, T, BT, OUT, 8, MRHS_CG> : k_sptrsv_mrhs<V, T, BT, OUT, 8, MRHS_CA>)
                            : (cg ? k_sptrsv_mrhs<V, T, BT, OUT, 16, MRHS_CG> : k_sptrsv_mrhs<V, T, BT, OUT, 16, MRHS_CA>);
         // the multi-RHS kernel takes at most 8 warps per block (its register use)
         const int mw = std::min(wpb, 8), mblock = 32 * mw;

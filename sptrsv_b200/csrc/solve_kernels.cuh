@@ -483,8 +483,71 @@ __device__ __forceinline__ void mrhs_load_round(const M& m, int s, int stride, i
     }
 }
 
-template <typename V, typename T, typename BT, int OUT, int U, int GM>
-__global__ void __launch_bounds__(256) k_sptrsv_mrhs(PermMat<V> m, int ntasks, const MrhsTask* __restrict__ tasks,
+// The same round with its entries spread over the row's lanes (kp >= U, whole
+// 16-byte copies): lane u of a row holds column c and value v of its entry u, and
+// the kp / VEC copies of an entry go to as many neighbouring lanes.
+template <typename T, int U>
+__device__ __forceinline__ bool mrhs_spread_round(int c, T v, int nh, const T* x, int K, int kp, int k, T* xs, int lane,
+                                                  T& acc, DevStatus* st, unsigned long long budget, unsigned backoff,
+                                                  int row)
+{
+    constexpr int VEC = 16 / sizeof(T);
+    const unsigned FULL = 0xffffffffu;
+    const int per = kp / VEC;  // copies of an entry
+    const int piece = (k & (per - 1)) * VEC, sub = k / per;
+    T* mine = xs + (lane - k) + piece;
+#pragma unroll
+    for (int j = 0; j < U / VEC; j++) {
+        const int u = j * VEC + sub;
+        const int cu = __shfl_sync(FULL, c, u, kp);
+        if (u < nh && piece < K) cp_async_cg16(mine + u * 32, x + (size_t)cu * K + piece);
+    }
+    cp_async_wait_all();
+    __syncwarp();
+    unsigned pend = 0;
+    if (k < K) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (u < nh && is_pending(xs[u * 32 + lane])) pend |= 1u << u;
+    }
+    unsigned any = __reduce_or_sync(FULL, pend), it = 0;
+    unsigned long long t0 = 0;
+    while (any) {
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (any >> u & 1u) {
+                const int cu = __shfl_sync(FULL, c, u, kp);
+                if (pend >> u & 1u) {
+                    const T w = ld_relaxed(x + (size_t)cu * K + k);
+                    if (!is_pending(w)) {
+                        xs[u * 32 + lane] = w;
+                        pend &= ~(1u << u);
+                    }
+                }
+            }
+        any = __reduce_or_sync(FULL, pend);
+        ++it;
+        if (backoff && it > 8 && any) __nanosleep(backoff);
+        if ((it & 63u) == 0 && any && give_up(t0, st, budget, row)) return false;
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        const T vu = __shfl_sync(FULL, v, u, kp);
+        if (u < nh && k < K) acc -= vu * xs[u * 32 + lane];
+    }
+    __syncwarp();  // the slots are reused by the next round
+    return true;
+}
+
+// SPREAD: a lane that keeps the U columns and values of its row's round, the same
+// in all of the row's lanes, takes 128 registers, 16 warps an SM; spread over
+// them 64, and twice the gathers are in flight (Zipf n = 2e6, 24 entries a row:
+// 16 right-hand sides 3.49 -> 2.7 ms, 32 6.8 -> 5.1 ms, refined 14.4 -> 11.1 and
+// 26.4 -> 19.0 ms).  The shuffles that hand them out lengthen a hop: short rows
+// and narrow levels keep the other form (101 x 90 x 97, 16: 611 against 690 us;
+// banded n = 5e4 in 1000: 900 against 1125 us).
+template <typename V, typename T, typename BT, int OUT, int U, int GM, bool SPREAD = false>
+__global__ void __launch_bounds__(256, SPREAD ? 4 : 0) k_sptrsv_mrhs(PermMat<V> m, int ntasks, const MrhsTask* __restrict__ tasks,
                                                      int K, int kp, const BT* __restrict__ b, T* x, double* x64,
                                                      T* pbuf, int* pcnt, DevStatus* st, unsigned long long budget,
                                                      unsigned backoff)
@@ -509,10 +572,20 @@ __global__ void __launch_bounds__(256) k_sptrsv_mrhs(PermMat<V> m, int ntasks, c
     mrhs_lane_range(h, h2, seg, E, s, n, stride);
     int rr = __ldg(m.rowid + (h.y > 0 ? h.x + min(seg, h.y - 1) : h.x));
     T piv = (T)__ldg(m.di + (h.y > 0 ? h.x + min(seg, h.y - 1) : h.x));
-    int cc[U];
-    T vv[U];
-    int nh = kok ? min(U, n) : 0;
-    mrhs_load_round<PermMat<V>, T, U>(m, s, stride, nh, cc, vv);
+    int cc[SPREAD ? 1 : U];
+    T vv[SPREAD ? 1 : U];
+    int nh;
+    // the first round (SPREAD: the one from entry j on, lane u of a row taking entry u)
+    auto load_round = [&](int j) {
+        if constexpr (SPREAD) {
+            nh = max(0, min(U, n - j));
+            mrhs_load_round<PermMat<V>, T, 1>(m, s + (j + k) * stride, stride, k < nh, cc, vv);
+        } else {
+            nh = kok ? min(U, n) : 0;
+            mrhs_load_round<PermMat<V>, T, U>(m, s, stride, nh, cc, vv);
+        }
+    };
+    load_round(0);
     while (true) {
         const int tn = t + nw;
         int4 g = h, g2 = h2;
@@ -525,14 +598,23 @@ __global__ void __launch_bounds__(256) k_sptrsv_mrhs(PermMat<V> m, int ntasks, c
         const size_t xi = (size_t)rr * K + k;
         const T bval = out ? (T)b[xi] : (T)0;  // used at publish time
         T acc = 0;  // minus the sum of this lane's products
-        mrhs_gather<T, U, GM>(cc, nh, xk, K, k, xs, lane);
-        if (!mrhs_finish_round<T, U>(cc, vv, nh, xk, K, xs, lane, acc, st, budget, backoff, rr)) return;
-        // later rounds (pieces cut longer than one round), loaded on the spot
-        for (int j = U; __any_sync(FULL, kok && j < n); j += U) {
-            const int mh = kok ? max(0, min(U, n - j)) : 0;
-            mrhs_load_round<PermMat<V>, T, U>(m, s + j * stride, stride, mh, cc, vv);
-            mrhs_gather<T, U, GM>(cc, mh, xk, K, k, xs, lane);
-            if (!mrhs_finish_round<T, U>(cc, vv, mh, xk, K, xs, lane, acc, st, budget, backoff, rr)) return;
+        // later rounds (pieces cut longer than one round) are loaded on the spot
+        if constexpr (SPREAD) {
+            for (int j = U;; j += U) {
+                if (!mrhs_spread_round<T, U>(cc[0], vv[0], nh, x, K, kp, k, xs, lane, acc, st, budget, backoff, rr))
+                    return;
+                if (!__any_sync(FULL, j < n)) break;
+                load_round(j);
+            }
+        } else {
+            mrhs_gather<T, U, GM>(cc, nh, xk, K, k, xs, lane);
+            if (!mrhs_finish_round<T, U>(cc, vv, nh, xk, K, xs, lane, acc, st, budget, backoff, rr)) return;
+            for (int j = U; __any_sync(FULL, kok && j < n); j += U) {
+                const int mh = kok ? max(0, min(U, n - j)) : 0;
+                mrhs_load_round<PermMat<V>, T, U>(m, s + j * stride, stride, mh, cc, vv);
+                mrhs_gather<T, U, GM>(cc, mh, xk, K, k, xs, lane);
+                if (!mrhs_finish_round<T, U>(cc, vv, mh, xk, K, xs, lane, acc, st, budget, backoff, rr)) return;
+            }
         }
         if (group) {
             if (out) publish<T, OUT>(x, x64, xi, (bval + acc) * piv);
@@ -570,8 +652,7 @@ __global__ void __launch_bounds__(256) k_sptrsv_mrhs(PermMat<V> m, int ntasks, c
         const int rpos = h.y > 0 ? h.x + min(seg, h.y - 1) : h.x;
         rr = __ldg(m.rowid + rpos);
         piv = (T)__ldg(m.di + rpos);
-        nh = kok ? min(U, n) : 0;
-        mrhs_load_round<PermMat<V>, T, U>(m, s, stride, nh, cc, vv);
+        load_round(0);
     }
 }
 
