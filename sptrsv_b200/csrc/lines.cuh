@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(32 * kLineG, 1)
                 int c[U];
                 const int cnt = e - s - 1;
                 // the form that the analysis found, or the CSR has changed since
-                bool glob = false, bad = act && (cnt < 0 || cnt > U || s < base || e - base > EC);
+                bool sub = false, glob = false, bad = act && (cnt < 0 || cnt > U || s < base || e - base > EC);
                 if (act && !bad) {
                     a = sb[buf * 32 + lane];
                     inv = 1.0 / sval[off + s + cnt];
@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(32 * kLineG, 1)
                         v[u] = sval[off + s + u];
                         if (c[u] == r - 1 && r > line0) {
                             lsub = v[u];
+                            sub = true;
                             c[u] = -1;
                         }
                         glob |= c[u] >= 0 && c[u] < R0;
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(32 * kLineG, 1)
                         if (c[u] >= 0 && c[u] < R0) xv[u] = ld_relaxed(x + c[u]);
                 }
                 // what does not depend on x
-                const double beta = -lsub * inv;
+                const double beta = sub ? -lsub * inv : 0.0;
                 const bool steep = __any_sync(FULL, !(fabs(beta) <= 1.0));
                 double M[5], B = beta;
 #pragma unroll
@@ -169,8 +170,7 @@ __global__ void __launch_bounds__(32 * kLineG, 1)
 #pragma unroll
                 for (int u = 0; u < U; u++)
                     if (c[u] >= 0) a -= v[u] * xv[u];
-                a *= inv;
-                double A = a;
+                double A = a * inv;
                 if (lane == 0) A += beta * carry;
 #pragma unroll
                 for (int d = 0; d < 5; d++) {
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(32 * kLineG, 1)
                 if (__any_sync(FULL, !finite_bits(A)) || steep) {
                     double t = carry;
                     for (int l = 0; l < 32; l++) {
-                        t = a + beta * t;
+                        t = (sub ? a - lsub * t : a) * inv;
                         if (lane == l) A = publishable(t);
                         t = __shfl_sync(FULL, t, l);
                     }

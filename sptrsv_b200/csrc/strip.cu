@@ -210,14 +210,15 @@ namespace {
 // bad |= 1 where a row has more than one entry beside the one on the row before,
 // or that one lies inside the row's chunk, or the row before counts for more
 // than the row itself (a scan over 128 rows multiplies these factors: they must
-// not grow).  pub[q] = 1 for chunks that another group reads.
+// not grow), or the row's reciprocal diagonal is not finite (0 times it is not
+// 0).  pub[q] = 1 for chunks that another group reads.
 __global__ void k_wave4_check(SptLayout l, const int* __restrict__ inv, int n, const int* __restrict__ rchunk,
                               const int* __restrict__ cstart, const int* __restrict__ cgroup, int* pub, int* bad)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int q = rchunk[i], p = inv[i];
         int cnt = 0;
-        bool no = false;
+        bool no = !isfinite(l.di64[p]) || !isfinite(l.di32[p]);
         for (int t = l.ptr[p]; t < l.ptr[p + 1]; t++) {
             const int c = l.col[t];
             if (c == i - 1) {
