@@ -73,14 +73,16 @@ def f32_launch_bytes(n: int, nnz: int, k: int) -> int:
     return 4 * (n + 1) + 4 * n + 4 * n + 8 * (nnz - n) + 8 * n * k + 4 * n * k
 
 
-def solve_launches(sched, mode: int, ir_iters: int) -> int:
-    """Kernels of the library launched per solve: the solve kernel, plus a
-    gather of b into the block system and a scatter of x out of it when
-    partitioned (BAND writes x itself), plus b into BAND's records; FP32 +
-    refinement adds a residual and another solve per step."""
+def solve_launches(sched, mode: int, ir_iters: int, own_rows: bool = False) -> int:
+    """Kernels of the library launched per solve, counted for the general form:
+    the solve kernel, plus a gather of b into the block system and a scatter
+    of x out of it when partitioned; two for BAND.  own_rows: the solve kernel
+    alone, as it reads b and writes x in the plan's rows (BAND; WAVE on blocks
+    of a 2D stencil).  FP32 + refinement adds a residual and another solve per
+    step."""
     band = sched.variant == 6
     part = sched.partitions >= 2
-    one = 2 if band else (3 if part else 1)
+    one = 1 if own_rows else 2 if band else (3 if part else 1)
     return one if mode == 64 else one * (1 + ir_iters) + ir_iters
 
 
@@ -583,7 +585,9 @@ def run_ours(args, rank, world, local, dist):
     total_ms = reduce_max(dist, sum(ts))
     value = world * k * args.steps / (total_ms / 1e3)
     ms_per_step = total_ms / args.steps
-    launches_per_step = solve_launches(SEL.schedule_from_class(sel64 if mode == 64 else sel32), mode, ir_iters)
+    picked = SEL.schedule_from_class(sel64 if mode == 64 else sel32)
+    launches_per_step = solve_launches(picked, mode, ir_iters, k == 1 and (
+        picked.variant == 6 or (picked.variant == 5 and args.config == "c1")))
 
     # --- the other mode and the drop-in FP64 path
     other = 32 if mode == 64 else 64

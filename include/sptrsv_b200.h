@@ -212,9 +212,9 @@ typedef struct sptrsv_plan_s* sptrsv_plan_t;
 #define SPTRSV_VAR_WAVE      5  /* STRIP's chunks; block_warps grid lines per CTA,   */
                                 /* one warp per line, the lines' x in shared memory  */
                                 /* (their rows must fit: 25,600 rows in FP64)        */
-#define SPTRSV_VAR_BAND      6  /* one warp per independent unit (the matrix, or a  */
-                                /* block of a partitioned schedule), level by level, */
-                                /* x in a shared-memory ring, no cross-warp waits;   */
+#define SPTRSV_VAR_BAND      6  /* one CTA per independent unit (the matrix, or a   */
+                                /* block of a partitioned schedule), step by step,   */
+                                /* x in shared memory, no waits on other CTAs;       */
                                 /* rows of at most 128 off-diagonals, levels of at   */
                                 /* most 128 rows on average per unit                 */
 #define SPTRSV_N_VARIANTS    7
@@ -310,7 +310,7 @@ int sptrsv_residual_f64(sptrsv_plan_t plan, const double* b, const double* x, do
  * memory when they solve — code whose device heap is owned by a pool or an
  * arena, or that must not call cudaMalloc after start-up.  The caller passes
  * the device CSR (diagonal last), b and x (DEVICE, n values); no analysis or
- * plan is needed.  FP32 solve in natural-order chunks, then ir_iters
+ * plan is needed.  FP32 solve in natural-order groups, then ir_iters
  * (0..16; others give SPTRSV_ERR_INVALID_ARG) refinement steps (FP64
  * residual, FP32 correction, x += d in FP64).  The CSR is not checked on the
  * host: the kernels check every row range and column before they use it, and

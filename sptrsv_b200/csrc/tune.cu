@@ -49,7 +49,7 @@ int sptrsv_schedule_from_class(int cls, sptrsv_schedule_t* s)
             {SPTRSV_VAR_MULTIROW, 1, 8, 0, 0, 64, 4096, 0},  {SPTRSV_VAR_MULTIROW, 1, 8, 0, 200, 64, 4096, 0},
             {SPTRSV_VAR_MULTIROW, 1, 4, 16, 0, 64, 4096, 0}, {SPTRSV_VAR_MULTIROW, 1, 16, 0, 0, 64, 4096, 0},
             {SPTRSV_VAR_MULTIROW, 1, 8, 0, 0, 64, 4096, 16}, {SPTRSV_VAR_MULTIROW, 1, 8, 0, 0, 64, 4096, 128},
-            // CLUSTER (bands of H levels cut into clusters of B rows) and BAND (one warp per unit), whole and
+            // CLUSTER (bands of H levels cut into clusters of B rows) and BAND (one CTA per unit), whole and
             // over blocks with warm-ups
             {SPTRSV_VAR_CLUSTER, 16, 16, 0, 0, 256, 2048, 0}, {SPTRSV_VAR_CLUSTER, 16, 8, 0, 0, 4096, 2048, 0},
             {SPTRSV_VAR_BAND, 1, 8, 0, 0, 64, 4096, 0},       {SPTRSV_VAR_CLUSTER, 16, 16, 0, 0, 256, 2048, 16},
