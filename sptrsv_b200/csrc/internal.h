@@ -185,7 +185,7 @@ struct AnalysisRec {
     int* d_wlev = nullptr;     // [n_warps]
     int* d_lptr = nullptr;     // [nlevs+1] first iorder position of each level
     int stats[20] = {};        // level widths and row lengths (k_level_sizes), grid lines (k_line_check)
-    int* slab[3] = {};         // the allocations that hold these arrays and the info struct's
+    int* slab[5] = {};         // the allocations that hold these arrays and the info struct's
     bool map_in_info = false;  // map arrays are also referenced by the info struct
     int* tile_tasks[6] = {};   // level-aligned iorder tasks for 32>>j lanes per row
     int tile_ntasks[6] = {};
