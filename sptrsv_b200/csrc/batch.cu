@@ -392,19 +392,24 @@ __device__ __forceinline__ void seq_unit(const SeqSet& q, const V* __restrict__ 
                         a2 += (nm > 1 ? e1.v : (T)0) * x1;
                         a3 += (nm > 2 ? e2.v : (T)0) * x2;
                         e += nm;
-                    } else {  // nothing to wait for
-                        asm volatile("barrier.cta.arrive %0, 64;" ::"r"(8 + tw) : "memory");
                     }
                 }
                 const T acc = (a0 + a1) + (a2 + a3);
+                // A row without such entries waits for that hand-over all the same, before its turn.  If
+                // its warp only arrived there, it could come to the barrier again, for row r + W, before
+                // row r - H's warp has issued its arrival (that comes after the hand-over to row
+                // r - H + 1, so nothing orders it): the barrier would open with this warp's two arrivals.
+                const bool owe = halves && r - H >= r0 && nm == 0;
                 if (nl == 0) {
                     res = acc * piv;
                     if (lk) *slot = res;
+                    if (owe) asm volatile("barrier.cta.sync %0, 64;" ::"r"(8 + tw) : "memory");
                     if (turn) asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + tw) : "memory");
                 } else {
                     const SeqEntry<T> e0 = e[0], e1 = e[nl > 1 ? 1 : 0], e2 = e[nl > 2 ? 2 : 0];
                     const T v1 = nl > 1 ? e1.v : (T)0, v2 = nl > 2 ? e2.v : (T)0;
                     *sum = acc;  // through memory, so that its arithmetic is done before the turn
+                    if (owe) asm volatile("barrier.cta.sync %0, 64;" ::"r"(8 + tw) : "memory");
                     if (turn) asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + tw) : "memory");
                     const T x0 = mine[e0.at], x1 = mine[e1.at], x2 = mine[e2.at];
                     T t = *sum;
@@ -415,7 +420,7 @@ __device__ __forceinline__ void seq_unit(const SeqSet& q, const V* __restrict__ 
                     if (lk) *slot = res;
                 }
             } else {  // everything in the row's turn
-                if (halves && r - H >= r0) asm volatile("barrier.cta.arrive %0, 64;" ::"r"(8 + tw) : "memory");
+                if (halves && r - H >= r0) asm volatile("barrier.cta.sync %0, 64;" ::"r"(8 + tw) : "memory");
                 if (turn) asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + tw) : "memory");
                 T t = b1;
                 for (int k = 0; k < n; k++) {
