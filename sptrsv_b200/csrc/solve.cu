@@ -559,8 +559,13 @@ int plan_launch(sptrsv_plan_s* p, bool f32, const BT* b, T* x, double* x64, int 
     if (sc.variant == SPTRSV_VAR_WAVE && nrhs == 1) {
         int e = build_wave_layout(p, sc.block_warps, kWaveMaxRows);
         if (e) return e;
-        if constexpr (sizeof(V) == 8 && OUT == OUT_X)  // only a streamed host solve comes here with this layout
-            if (p->wave4.chunk) return launch_wave4<V, T, BT, OUT, true>(p, b, nullptr, nullptr, s);
+        if (p->wave4.chunk) {
+            // only a streamed host solve comes here with this layout: the others launch it from the outer
+            // plan (part_wave4), with the vectors of its rows
+            if constexpr (sizeof(V) == 8 && OUT == OUT_X)
+                if (p->launch_hx) return launch_wave4<V, T, BT, OUT, true>(p, b, nullptr, nullptr, s);
+            return set_error(SPTRSV_ERR_UNSUPPORTED, "wave: a block system's layout needs its outer plan");
+        }
     }
     // the kernels below wait on x itself: not ready is all ones
     SPT_CUDA(cudaMemsetAsync(x, 0xFF, sizeof(T) * (size_t)n * nrhs, s));
@@ -737,6 +742,17 @@ int part_own_rhs(sptrsv_plan_s* p, const BT* b, const X* x, cudaStream_t s, cons
     return 0;
 }
 
+// *yes: the block system is solved by its wave4 layout.  Builds the schedule's
+// layout first: a schedule that was refused may have taken it away.
+int part_wave4(PartPlan* q, int nrhs, bool* yes)
+{
+    *yes = false;
+    if (nrhs != 1 || q->sub->sched.variant != SPTRSV_VAR_WAVE) return 0;
+    int e = build_wave_layout(q->sub, q->sub->sched.block_warps, kWaveMaxRows);
+    *yes = !e && q->sub->wave4.chunk;
+    return e;
+}
+
 // Partitioned FP64 solve: b gathered into the block system, solved there,
 // each block's real rows scattered into x.
 int part_solve_f64(sptrsv_plan_s* p, const double* b, double* x, int nrhs, cudaStream_t s)
@@ -744,12 +760,15 @@ int part_solve_f64(sptrsv_plan_s* p, const double* b, double* x, int nrhs, cudaS
     PartPlan* q = p->part;
     if (q->sub->sched.variant == SPTRSV_VAR_BAND && nrhs == 1)  // records map to this plan's rows
         return band_solve(q->sub, false, b, false, x, nullptr, OUT_X, s);
-    if (nrhs == 1 && q->sub->sched.variant == SPTRSV_VAR_WAVE && q->sub->wave4.chunk) {
-        int e = part_own_rhs(p, b, x, s, &b);
+    bool wave4;
+    int e = part_wave4(q, nrhs, &wave4);
+    if (e) return e;
+    if (wave4) {
+        e = part_own_rhs(p, b, x, s, &b);
         if (e) return e;
         return launch_wave4<double, double, double, OUT_X, false>(q->sub, b, x, nullptr, s);
     }
-    int e = part_ensure(q, nrhs);
+    e = part_ensure(q, nrhs);
     if (!e) e = part_gather64(q, b, q->bx, nrhs, s);
     if (!e) e = plan_solve_f64(q->sub, q->bx, q->xx, nrhs, s);
     if (!e) e = part_scatter64(q, q->xx, x, nrhs, s);
@@ -762,8 +781,11 @@ int part_solve32(sptrsv_plan_s* p, const BT* rhs, float* out32, double* x64, int
     PartPlan* q = p->part;
     if (q->sub->sched.variant == SPTRSV_VAR_BAND && nrhs == 1)
         return band_solve(q->sub, true, rhs, sizeof(BT) == 4, out32, x64, out_mode, s);
-    if (nrhs == 1 && q->sub->sched.variant == SPTRSV_VAR_WAVE && q->sub->wave4.chunk) {
-        int e = out_mode == OUT_X ? part_own_rhs(p, rhs, out32, s, &rhs) : part_own_rhs(p, rhs, x64, s, &rhs);
+    bool wave4;
+    int e = part_wave4(q, nrhs, &wave4);
+    if (e) return e;
+    if (wave4) {
+        e = out_mode == OUT_X ? part_own_rhs(p, rhs, out32, s, &rhs) : part_own_rhs(p, rhs, x64, s, &rhs);
         if (e) return e;
         if (out_mode == OUT_SET64)
             return launch_wave4<float, float, BT, OUT_SET64, false>(q->sub, rhs, nullptr, x64, s);
@@ -771,7 +793,7 @@ int part_solve32(sptrsv_plan_s* p, const BT* rhs, float* out32, double* x64, int
             return launch_wave4<float, float, BT, OUT_ADD64, false>(q->sub, rhs, nullptr, x64, s);
         return launch_wave4<float, float, BT, OUT_X, false>(q->sub, rhs, out32, nullptr, s);
     }
-    int e = part_ensure(q, nrhs);
+    e = part_ensure(q, nrhs);
     if (e) return e;
     const BT* g;
     if constexpr (sizeof(BT) == 8) {
@@ -1183,7 +1205,8 @@ int sptrsv_solve_host(sptrsv_plan_t p, const double* hb, double* hx, int nrhs, i
         void* hx_dev = nullptr;
         if (nrhs == 1 && precision == 64 && p->sched.variant == SPTRSV_VAR_WAVE && mapped_host(hb) &&
             (hx_dev = mapped_host(hx)) != nullptr) {
-            int e = partitioned(p) ? 0 : build_wave_layout(p, p->sched.block_warps, kWaveMaxRows);
+            sptrsv_plan_s* lp = partitioned(p) ? p->part->sub : p;
+            int e = build_wave_layout(lp, lp->sched.block_warps, kWaveMaxRows);
             if (!e) e = solve_host_streamed(p, hb, (double*)hx_dev, s);
             if (e) return e;
             e = sync_status(s);
