@@ -351,6 +351,7 @@ __global__ void __launch_bounds__(kNatGroup, 3) k_sptrsv_natural(M m, int n, con
                             const int fin = __shfl_sync(FULL, (int)(ready && nl == 99), k);
                             if (fin && ready && nl == k) {
                                 acc -= nv * xk;
+                                inmask &= ~(1u << k);  // not again, should the warp turn out to hold an odd row
                                 next_in();
                             }
                         }
