@@ -177,7 +177,7 @@ int band_launch_t(const BandLayout& t, const unsigned char* rec, const BT* b, T*
 {
     auto kern = k_sptrsv_band<T, BT, OUT>;
     const size_t smem = (size_t)(t.R + 1) * sizeof(T);
-    if (smem > 32 * 1024) SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SPT_CUDA(allow_smem(kern, smem));
     kern<<<t.nunits, 32 * kBandWarps, smem, s>>>(rec, t.ustep, t.R, b, x, x64);
     SPT_CUDA(cudaGetLastError());
     return 0;

@@ -1292,8 +1292,7 @@ int vk_grid(const sptrsv_batch_s* B, bool sweep, long long max_blocks, long long
     const int cap = B->warps_per_sm > 0 ? (B->warps_per_sm + bw - 1) / bw : 0;
     const size_t smem = sweep ? sweep_per_block(B) * SweepSmem<V, T, BT>::total : SeqSmem<T>::total(seq_team(B));
     auto grid = [&](auto kern) -> int {
-        if (smem > 32 * 1024)  // the occupancy query needs the kernel's opt-in to large shared memory
-            SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SPT_CUDA(allow_smem(kern, smem));  // the occupancy query needs the kernel's opt-in to large shared memory
         SPT_CUDA(persistent_grid(kern, 32 * bw, smem, max_blocks, cap, g));
         return 0;
     };
@@ -1443,8 +1442,7 @@ int batch_launch(sptrsv_batch_s* B, bool f32, const BT* b, T* x, double* x64, cu
         SPT_CUDA(cudaMemsetAsync(B->flags, 0, sizeof(int) * (size_t)B->nchunks, s));
         auto kern = k_sptrsv_vkc<V, T, BT, OUT>;
         const size_t smem = (size_t)B->block_warps * 32 * 32 * sizeof(T);
-        if (smem > 32 * 1024)
-            SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SPT_CUDA(allow_smem(kern, smem));
         SPT_CUDA(launch_persistent_capped(kern, block, smem, div_up(B->nchunks, B->block_warps), cap, s, nb, val, di,
                                           B->nchunks, B->flags, b, x, x64, c->d_status, wait_budget_ns(),
                                           (unsigned)B->backoff_ns));
@@ -1464,8 +1462,7 @@ int batch_launch(sptrsv_batch_s* B, bool f32, const BT* b, T* x, double* x64, cu
     const int bw = B->sweep ? B->block_warps : vk_warps(B, B->nteams > 0);
     const int vcap = B->warps_per_sm > 0 ? (B->warps_per_sm + bw - 1) / bw : 0;
     auto go = [&](auto kern, auto bm) -> int {
-        if (smem > 32 * 1024)
-            SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        SPT_CUDA(allow_smem(kern, smem));
         SPT_CUDA(launch_persistent_capped(kern, 32 * bw, smem, vk_max_blocks(B, B->sweep, B->nteams), vcap, s, bm, val,
                                           di, B->ntasks, (const int*)B->tbase, (const int*)B->tkp, q, team, nval, ndi,
                                           b, x, x64, c->d_status, wait_budget_ns(), (unsigned)B->backoff_ns));

@@ -138,6 +138,20 @@ cudaError_t launch_persistent(void (*kern)(KArgs...), int block, size_t smem, lo
     return launch_persistent_capped(kern, block, smem, max_blocks, 0, s, args...);
 }
 
+// Opt-in to large dynamic shared memory, before the occupancy query and the
+// launch.  The default limit covers static plus dynamic shared memory up to 48 KB,
+// so a kernel with static shared memory needs the opt-in a little below that.
+// The limit belongs to the kernel, not to the launch: it is always set to the same
+// size, what an SM gives a CTA but for 3 KB of static shared memory.  Set to this
+// launch's size it could be lowered between another host thread's setting and launch.
+constexpr int kSmemLimit = 224 * 1024;
+template <typename K>
+cudaError_t allow_smem(K kern, size_t bytes)
+{
+    if (bytes <= 32 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
+}
+
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Grid for a plain grid-stride kernel: enough blocks for `work` threads,

@@ -43,16 +43,6 @@ size_t strip_smem_bytes(const sptrsv_schedule_t* s, size_t elem)
     return (size_t)s->block_warps * 2 * s->rows_per_warp * 32 * elem;
 }
 
-// Opt-in to large dynamic shared memory.  The default limit covers static
-// plus dynamic shared memory up to 48 KB, so a kernel with static shared
-// memory needs the opt-in a little below that.
-template <typename K>
-cudaError_t allow_smem(K kern, size_t bytes)
-{
-    if (bytes <= 32 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 __global__ void k_iorder_level_keys(const int* __restrict__ iorder, const int* __restrict__ level, int n,
                                     int* __restrict__ key)
 {
@@ -163,7 +153,7 @@ int launch_level_cta_kp(const M& m, const LevelCta& lc, bool ring, int g, const 
 {
     auto kern = ring ? k_sptrsv_level_cta<M, T, BT, OUT, KP, true> : k_sptrsv_level_cta<M, T, BT, OUT, KP, false>;
     const size_t smem = sizeof(T) * ((size_t)lc.slots + 1);
-    if (smem > 32 * 1024) SPT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SPT_CUDA(allow_smem(kern, smem));
     kern<<<1, 32 * kTeamWarps, smem, s>>>(m, lc, g, b, x, x64);
     SPT_CUDA(cudaGetLastError());
     return 0;
