@@ -375,9 +375,9 @@ __device__ __forceinline__ void seq_unit(const SeqSet& q, const V* __restrict__ 
                     a2 += e2.v * x2;
                     a3 += e3.v * x3;
                 }
-                if (rem) {
+                if (rem) {  // entries that are not there: 0 times the zero row (0 times an infinity is NaN)
                     const SeqEntry<T> e0 = e[0], e1 = e[rem > 1 ? 1 : 0], e2 = e[rem > 2 ? 2 : 0];
-                    const T x0 = mine[e0.at], x1 = mine[e1.at], x2 = mine[e2.at];
+                    const T x0 = mine[e0.at], x1 = mine[rem > 1 ? e1.at : zero], x2 = mine[rem > 2 ? e2.at : zero];
                     a1 += e0.v * x0;
                     a2 += (rem > 1 ? e1.v : (T)0) * x1;
                     a3 += (rem > 2 ? e2.v : (T)0) * x2;
@@ -387,7 +387,7 @@ __device__ __forceinline__ void seq_unit(const SeqSet& q, const V* __restrict__ 
                     if (nm) {
                         const SeqEntry<T> e0 = e[0], e1 = e[nm > 1 ? 1 : 0], e2 = e[nm > 2 ? 2 : 0];
                         asm volatile("barrier.cta.sync %0, 64;" ::"r"(8 + tw) : "memory");
-                        const T x0 = mine[e0.at], x1 = mine[e1.at], x2 = mine[e2.at];
+                        const T x0 = mine[e0.at], x1 = mine[nm > 1 ? e1.at : zero], x2 = mine[nm > 2 ? e2.at : zero];
                         a1 += e0.v * x0;
                         a2 += (nm > 1 ? e1.v : (T)0) * x1;
                         a3 += (nm > 2 ? e2.v : (T)0) * x2;
@@ -408,10 +408,11 @@ __device__ __forceinline__ void seq_unit(const SeqSet& q, const V* __restrict__ 
                 } else {
                     const SeqEntry<T> e0 = e[0], e1 = e[nl > 1 ? 1 : 0], e2 = e[nl > 2 ? 2 : 0];
                     const T v1 = nl > 1 ? e1.v : (T)0, v2 = nl > 2 ? e2.v : (T)0;
+                    const int at1 = nl > 1 ? e1.at : zero, at2 = nl > 2 ? e2.at : zero;
                     *sum = acc;  // through memory, so that its arithmetic is done before the turn
                     if (owe) asm volatile("barrier.cta.sync %0, 64;" ::"r"(8 + tw) : "memory");
                     if (turn) asm volatile("barrier.cta.sync %0, 64;" ::"r"(1 + tw) : "memory");
-                    const T x0 = mine[e0.at], x1 = mine[e1.at], x2 = mine[e2.at];
+                    const T x0 = mine[e0.at], x1 = mine[at1], x2 = mine[at2];
                     T t = *sum;
                     t += e0.v * x0;
                     t += v1 * x1;
