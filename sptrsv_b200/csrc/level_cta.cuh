@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(32 * kTeamWarps, 1) k_sptrsv_level_cta(M m, Le
                 }
             }
             const T piv = act ? (M::kInvStored ? ec.d : (T)1 / ec.d) : (T)0;
-            T acc = mine ? ec.b : (T)0;
+            const T rhs = mine ? ec.b : (T)0;
             const int p1 = cur.pos - first + (sub + G) * RPS;  // this warp's next rows of the level (uniform)
             const bool plain = __all_sync(0xffffffffu, n <= kTeamU && !far && p1 >= cur.end);
             const int own = own_slot(cur.r, cur.pos);
@@ -128,11 +128,14 @@ __global__ void __launch_bounds__(32 * kTeamWarps, 1) k_sptrsv_level_cta(M m, Le
             T xv[kTeamU];
 #pragma unroll
             for (int u = 0; u < kTeamU; u++) xv[u] = xs[cc[u]];
-            T acc1 = vv[1] * xv[1];
-            acc += vv[0] * xv[0];
-            acc1 += vv[3] * xv[3];
-            acc += vv[2] * xv[2];
-            acc += acc1;
+            auto sum = [&]() {
+                T s0 = rhs, s1 = vv[1] * xv[1];
+                s0 += vv[0] * xv[0];
+                s1 += vv[3] * xv[3];
+                s0 += vv[2] * xv[2];
+                return s0 + s1;
+            };
+            T acc = sum();
             if (plain) {
 #pragma unroll
                 for (int o = KP >> 1; o >= 1; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o, KP);
@@ -144,10 +147,11 @@ __global__ void __launch_bounds__(32 * kTeamWarps, 1) k_sptrsv_level_cta(M m, Le
                 if (!RING && mine) x[cur.r] = publishable(v);
                 if (mine) publish64(cur.r, v);
             } else {
-                if (RING) {  // columns that left the ring long ago
+                if (RING) {  // columns that left the ring long ago (summed anew: an infinity times the 0 above is NaN)
 #pragma unroll
                     for (int u = 0; u < kTeamU; u++)
-                        if (u < n && cc[u] == zero) acc += vv[u] * ld_relaxed(x + ec.c[u]);
+                        if (u < n && cc[u] == zero) xv[u] = ld_relaxed(x + ec.c[u]);
+                    if (far) acc = sum();
                 }
                 auto rest = [&](int p, int e) {  // entries beyond the ones loaded ahead
                     T t = (T)0;
