@@ -34,7 +34,7 @@
 // a free list and takes a slot back after its occupant's last reader (interval
 // allocation), so R = the most values alive at once (at most 8192); slot R
 // holds 0 for unused entries.  Where list scheduling keeps more than that
-// alive, the steps follow the levels.
+// alive, or needs more steps, the steps follow the levels (band_steps.h).
 #include <algorithm>
 #include <cstring>
 #include <exception>
@@ -42,6 +42,7 @@
 #include <thread>
 #include <vector>
 
+#include "band_steps.h"
 #include "internal.h"
 #include "plan.h"
 #include "solve_kernels.cuh"
@@ -51,7 +52,6 @@ namespace sptrsv {
 namespace {
 
 constexpr int kBandWarps = 8;     // one hardware barrier each
-constexpr int kBandMaxRing = 8192;
 
 // Record of one step: per lane a packet of 16-byte pieces, stored piece-major
 // (piece k of lane j at k * 512 + j * 16), so a warp reads a piece with one
@@ -183,109 +183,6 @@ int band_launch_t(const BandLayout& t, const unsigned char* rec, const BT* b, T*
     return 0;
 }
 
-// One step: rows [first, first + cnt) of the unit's step order, kp lanes each.
-struct BandStepHost {
-    int kp, first, cnt;
-};
-
-// The steps of one unit: rows [a, b) of the natural CSR, all of whose columns
-// lie in it, with their levels.
-struct BandUnit {
-    std::vector<BandStepHost> steps;
-    std::vector<int> order;    // rows in step order
-    std::vector<int> slot_of;  // by row - a
-    int R = 1;
-};
-
-int band_lanes(int len)
-{
-    int kp = 1;
-    while ((len + kp - 1) / kp > kBandU) kp *= 2;
-    return kp;
-}
-
-// List scheduling: of the rows whose columns lie in earlier steps, those with
-// the longest chain of readers first; the first one's lane count is the
-// step's, rows that need more wait.
-void band_list_steps(const int* rp, const int* ci, int a, int b, BandUnit& u)
-{
-    const int n = b - a;
-    std::vector<int> height(n, 0), missing(n), cptr(n + 1, 0);
-    int top = 0;
-    for (int r = b - 1; r >= a; r--) {
-        missing[r - a] = rp[r + 1] - 1 - rp[r];
-        top = std::max(top, height[r - a]);
-        for (int q = rp[r]; q < rp[r + 1] - 1; q++) {
-            int& h = height[ci[q] - a];
-            h = std::max(h, height[r - a] + 1);
-            cptr[ci[q] - a + 1]++;
-        }
-    }
-    for (int i = 0; i < n; i++) cptr[i + 1] += cptr[i];
-    std::vector<int> reader(cptr[n]), at(cptr.begin(), cptr.end() - 1);
-    for (int r = a; r < b; r++)
-        for (int q = rp[r]; q < rp[r + 1] - 1; q++) reader[at[ci[q] - a]++] = r;
-    std::vector<std::vector<int>> ready(top + 1);  // by height
-    for (int r = b - 1; r >= a; r--)
-        if (missing[r - a] == 0) ready[height[r - a]].push_back(r);
-    u.steps.clear();
-    u.order.clear();
-    u.order.reserve(n);
-    std::vector<int> wait;
-    int hi = top;
-    while ((int)u.order.size() < n) {
-        while (ready[hi].empty()) hi--;
-        const int first = (int)u.order.size();
-        int kp = 0, per = 0;
-        for (int h = hi; h >= 0; h--) {
-            wait.clear();
-            while (!ready[h].empty() && (kp == 0 || (int)u.order.size() - first < per)) {
-                const int r = ready[h].back();
-                ready[h].pop_back();
-                const int need = band_lanes(rp[r + 1] - 1 - rp[r]);
-                if (kp == 0) {
-                    kp = need;
-                    per = 32 / kp;
-                }
-                if (need > kp) wait.push_back(r);
-                else u.order.push_back(r);
-            }
-            for (size_t k = wait.size(); k-- > 0;) ready[h].push_back(wait[k]);
-            if ((int)u.order.size() - first >= per) break;
-        }
-        const int cnt = (int)u.order.size() - first;
-        u.steps.push_back({kp, first, cnt});
-        for (int k = first; k < first + cnt; k++) {
-            const int i = u.order[k] - a;
-            for (int q = cptr[i]; q < cptr[i + 1]; q++) {
-                const int r = reader[q];
-                if (--missing[r - a] == 0) {
-                    ready[height[r - a]].push_back(r);
-                    hi = std::max(hi, height[r - a]);
-                }
-            }
-        }
-    }
-}
-
-// Steps along the levels: every level cut by itself, its lane count from its
-// longest row.
-void band_level_steps(const int* rp, const int* lev, int a, int b, BandUnit& u)
-{
-    u.steps.clear();
-    u.order.resize(b - a);
-    for (int r = a; r < b; r++) u.order[r - a] = r;
-    std::stable_sort(u.order.begin(), u.order.end(), [&](int p, int q) { return lev[p] < lev[q]; });
-    for (int f = 0; f < b - a;) {
-        int e = f, mx = 0;
-        for (; e < b - a && lev[u.order[e]] == lev[u.order[f]]; e++)
-            mx = std::max(mx, rp[u.order[e] + 1] - 1 - rp[u.order[e]]);
-        const int kp = band_lanes(mx), per = 32 / kp;
-        for (int q = f; q < e; q += per) u.steps.push_back({kp, q, std::min(per, e - q)});
-        f = e;
-    }
-}
-
 // f(0 .. n-1) over the host's threads; what a thread throws is thrown here,
 // once all of them have ended.
 template <class F>
@@ -312,43 +209,6 @@ void band_spread(int n, F&& f)
     for (auto& x : th) x.join();
     for (auto& e : err)
         if (e) std::rethrow_exception(e);
-}
-
-// Slots by interval allocation over the steps; false when more than
-// kBandMaxRing values are alive at once.
-bool band_slots(const int* rp, const int* ci, int a, int b, BandUnit& u)
-{
-    const int n = b - a, ns = (int)u.steps.size();
-    std::vector<int> last(n, -1), step(n);
-    for (int t = 0; t < ns; t++)
-        for (int k = u.steps[t].first; k < u.steps[t].first + u.steps[t].cnt; k++) {
-            const int r = u.order[k];
-            step[r - a] = t;
-            for (int q = rp[r]; q < rp[r + 1] - 1; q++) last[ci[q] - a] = t;  // steps ascend
-        }
-    std::vector<int> rptr(ns + 1, 0);
-    for (int i = 0; i < n; i++) rptr[std::max(last[i], step[i]) + 1]++;
-    for (int t = 0; t < ns; t++) rptr[t + 1] += rptr[t];
-    std::vector<int> rel(n), at(rptr.begin(), rptr.end() - 1), freel;
-    u.slot_of.assign(n, 0);
-    int top = 0;
-    for (int t = 0; t < ns; t++) {
-        for (int k = u.steps[t].first; k < u.steps[t].first + u.steps[t].cnt; k++) {
-            const int i = u.order[k] - a;
-            int sl;
-            if (!freel.empty()) {
-                sl = freel.back();
-                freel.pop_back();
-            } else {
-                sl = top++;
-            }
-            u.slot_of[i] = sl;
-            rel[at[std::max(last[i], t)]++] = sl;
-        }
-        for (int k = rptr[t]; k < rptr[t + 1]; k++) freel.push_back(rel[k]);  // free from the next step on
-    }
-    u.R = std::max(1, top);
-    return u.R <= kBandMaxRing;
 }
 
 }  // namespace
@@ -409,11 +269,7 @@ int build_band_layout(sptrsv_plan_s* p)
     auto spread = [&](auto&& f) { band_spread(nunits, f); };
     spread([&](int un) {
         const int a = u0[un], b = u0[un + 1];
-        band_list_steps(rp.data(), ci.data(), a, b, units[un]);
-        if (!band_slots(rp.data(), ci.data(), a, b, units[un])) {
-            band_level_steps(rp.data(), lev.data(), a, b, units[un]);
-            band_slots(rp.data(), ci.data(), a, b, units[un]);
-        }
+        band_unit(rp.data(), ci.data(), lev.data(), a, b, units[un]);
     });
     int R = 1;
     std::vector<int> ustep(nunits + 1, 0);

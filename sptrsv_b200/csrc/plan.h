@@ -115,7 +115,6 @@ struct MrhsTable {
 // BAND schedule (built on demand, see band.cu): per unit (the whole matrix,
 // or each block of a block system) its steps as fixed-size records, FP64 and
 // FP32 copies.
-constexpr int kBandU = 4;  // entries per lane per step
 struct BandLayout {
     int U = 0, R = 0;          // entries per lane per step; ring slots (slot R is a constant 0)
     int nunits = 0, nsteps = 0;
