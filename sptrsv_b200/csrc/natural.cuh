@@ -15,8 +15,9 @@
 //     affine prefix scan over the lanes into which the row before the warp
 //     enters last.  Lanes that start a new grid line start a new segment of
 //     the scan, and a segment is closed as soon as its own rows are known:
-//     one line's end does not hold up the next line's start.  A result that
-//     is not finite sends the warp to the general form below;
+//     one line's end does not hold up the next line's start.  A row is always
+//     of the same scan over its segment, whichever rows were known together;
+//     rows that are not finite by it are taken one after another;
 //   * otherwise one pass over the lanes that are read, in order, broadcasts
 //     each value to the rows that read it, once all of the warp's outside
 //     columns are known or, as far as it goes, when some are long in coming;
@@ -29,9 +30,9 @@
 // far from the front costs one sector a poll.
 //
 // Bound: the hops.  FP64 solves before and after (a warp took 32 rows one after
-// another): 1000 x 900 grid 444 -> 1.3 ms, 101 x 90 x 97 grid 543 -> 0.74 ms,
-// Zipf n = 1e6 39.6 -> 2.2 ms, banded n = 1e5 55.5 -> 8.8 ms, dense 32-row
-// blocks n = 3e5 65 -> 47 us.
+// another): 1000 x 900 grid 444 -> 1.2 ms, 101 x 90 x 97 grid 543 -> 0.69 ms,
+// Zipf n = 1e6 39.6 -> 2.1 ms, banded n = 1e5 55.5 -> 8.9 ms, dense 32-row
+// blocks n = 3e5 74 -> 49 us.
 //
 // STAGE: the entries of a warp's 32 rows are contiguous in the caller's CSR; up
 // to kNatStage of them are copied to shared memory by coalesced cp.async, as
@@ -175,17 +176,18 @@ __global__ void __launch_bounds__(kNatGroup, 3) k_sptrsv_natural(M m, int n, con
         if (CHECK) fail = __any_sync(FULL, fail);
 
         const bool sub = lane > 0 && (inmask >> (lane - 1) & 1u);
-        T beta = (T)0;      // factor of the row before, where the recurrence continues it
+        T lsub = (T)0, beta = (T)0;  // the row before: its entry, its factor where the recurrence continues it
         unsigned cinbit = 0;  // lane 0: the column that is the row before the warp
         int far = -1;
 #pragma unroll
         for (int u = 0; u < kNatU; u++)
             if (u < min(nb, kNatU) && c[u] == r - 1) {
-                beta = -v[u] * piv;
+                lsub = v[u];
+                beta = -lsub * piv;
                 if (lane == 0) cinbit = 1u << u;
             }
         const bool single = __popc(inmask) == (q.e - p - __popc(outside));  // no column inside the warp twice
-        bool chain = __all_sync(FULL, q.e - p <= kNatU && inmask == (sub ? 1u << (lane - 1) : 0u) && single &&
+        const bool chain = __all_sync(FULL, q.e - p <= kNatU && inmask == (sub ? 1u << (lane - 1) : 0u) && single &&
                                           fabs((double)beta) <= 1.0 && __popc(cinbit) <= 1);
         if (!chain) cinbit = 0;
 #pragma unroll
@@ -230,10 +232,10 @@ __global__ void __launch_bounds__(kNatGroup, 3) k_sptrsv_natural(M m, int n, con
             xs[tid] = val;
             publish<T, OUT>(x, x64, (size_t)q.r, val);
             done = true;
-            acc = val;  // what the rows inside the warp that read it take
+            if (chain) return;  // later scans of the warp take the row as this one did
+            acc = val;          // what the rows inside the warp that read it take
             piv = (T)1;
             nl = 99;
-            beta = (T)0;  // later scans of the warp start here
         };
         bool all = true, stalled = false, walking = false;
         while (!fail) {
@@ -290,28 +292,21 @@ __global__ void __launch_bounds__(kNatGroup, 3) k_sptrsv_natural(M m, int n, con
                 const T in = __shfl_sync(FULL, vin, 0);
                 const bool hang = start == 0 && cin;  // the segment hangs on the row before the warp
                 const bool now = !done && (R & need) == need && (!hang || known);
-                const T val = hang ? A + B * in : A;
+                const T val = hang ? A + B * in : A;  // of the same scan whatever other rows were ready
+                T fin = val;
                 if (__any_sync(FULL, now && !isfinite(val))) {
-                    chain = false;  // in order below, as infinities and NaN spread there
-                    if (cinbit && !done) {
-                        if ((pend & cinbit) == 0) {
-#pragma unroll
-                            for (int u = 0; u < kNatU; u++)
-                                if (cinbit >> u & 1u) acc -= v[u] * xv[u];
-                            outside &= ~cinbit;
-                        } else if (ready) {  // the round is subtracted but for this column
-                            ready = false;
-                            outside = pend = cinbit;
-                            p = q.s;
-                            nb = q.e - q.s;
+                    // such rows one after another, as infinities and NaN spread in substitution; a
+                    // row whose scan is finite has only finite ones before it in its segment
+                    T t = in;
+                    for (int k = 0; k < 32; k++) {
+                        if (lane == k) {
+                            if (done) fin = xs[tid];
+                            else if (!isfinite(val)) fin = publishable((sub || cinbit ? acc - lsub * t : acc) * piv);
                         }
+                        t = __shfl_sync(FULL, fin, k);
                     }
-                    cinbit = 0;
-                    seen = 0;
-                    all = true;
-                    continue;
                 }
-                if (now) finish(val);
+                if (now) finish(fin);
             } else {
                 const bool full = R == FULL;
                 if (full || (stalled && R != seen)) {
