@@ -19,9 +19,13 @@
 //  4. Multirow warp map [:354-385, kernel_base :244-270]: warps per key =
 //     ceil(count * lanes / 32), two exclusive scans, then one thread per warp
 //     writes ibase_row / ivect_size_warp.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
+#include <vector>
 
+#include "blocks.h"
 #include "internal.h"
 
 namespace sptrsv {
@@ -429,6 +433,37 @@ __global__ void k_inverse(const int* __restrict__ perm, int n, int* __restrict__
 
 
 
+struct Place {
+    int** p;
+    long long ints;
+};
+
+// Device arrays, in one allocation or one each (share_block); the allocations are
+// added to blocks.
+cudaError_t place(std::vector<int*>& blocks, long long small, std::initializer_list<Place> arrays)
+{
+    std::vector<long long> ints;
+    long long sum = 0;
+    for (const Place& a : arrays) {
+        ints.push_back(std::max<long long>(1, a.ints));
+        sum += block_part(ints.back());
+    }
+    const bool share = share_block(ints.data(), (int)ints.size(), small);
+    int* at = nullptr;
+    int k = 0;
+    for (const Place& a : arrays) {
+        const long long n = block_part(ints[k++]);
+        if (!at) {
+            cudaError_t e = dalloc(&at, share ? sum : n);
+            if (e != cudaSuccess) return e;
+            blocks.push_back(at);
+        }
+        *a.p = at;
+        at = share ? at + n : nullptr;
+    }
+    return cudaSuccess;
+}
+
 }  // namespace
 
 // Checks a device CSR; returns 0, SPTRSV_ERR_INVALID_CSR (with *bad_row) or a CUDA error code.
@@ -465,17 +500,14 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     cudaStream_t s = 0;
     const int nnz = L->nnz;
 
-    // A device allocation and its release cost about 0.1 ms each, whatever
-    // their size, so the arrays share four: what n alone sizes, scratch, what
-    // the level count sizes, and the warp map.
     AnalysisRec* rec = new AnalysisRec();
     rec->device = c->device;
     rec->n = n;
     rec->nnz = nnz;
-    int* scratch = nullptr;
+    std::vector<int*> scratch;  // its allocations
     auto fail = [&](int code) {
-        cudaFree(scratch);
-        for (int* q : rec->slab) cudaFree(q);
+        free_blocks(scratch);
+        free_blocks(rec->slab);
         delete rec;
         return code;
     };
@@ -484,21 +516,12 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
         cudaError_t e_ = (call);                                \
         if (e_ != cudaSuccess) return fail(cuda_fail(e_, #call)); \
     } while (0)
-    auto part = [](long long ints) { return (ints + 63) / 64 * 64; };  // 256-byte aligned
-    const long long pn = part(n);
-    // Arrays that the driver takes from its small blocks stay apart where their sum would not be
-    // (1e5 rows in blocks of 32: 1.0 ms apart, 1.7 ms together; 1.3e5: 1.6 either way).
-    const bool apart = n > 65536 && n <= 150000;
-    ACHK(dalloc(&rec->slab[0], (apart ? 1 : 3) * pn + 64));
-    if (apart)
-        for (int k = 3; k < 5; k++) ACHK(dalloc(&rec->slab[k], pn));
-    int* d_rowctr = rec->slab[0];
+    int *d_rowctr, *d_iorder, *d_inv, *d_key, *d_key2, *d_val2, *d_scr;
+    ACHK(place(rec->slab, kRowShare, {{&d_rowctr, n + 64LL}, {&d_iorder, n}, {&d_inv, n}}));
     rec->d_levels = d_rowctr + 64;
-    int *d_iorder = apart ? rec->slab[3] : rec->d_levels + pn, *d_inv = apart ? rec->slab[4] : d_iorder + pn;
-    const long long scr = radix_scratch_ints(n), keys = 3 * pn;
-    ACHK(dalloc(&scratch, keys + part(scr) + 64));
-    int *d_key = scratch, *d_key2 = d_key + pn, *d_val2 = d_key2 + pn, *d_scr = d_val2 + pn;
-    int* d_nlevs = d_scr + part(scr);
+    const long long scr = block_part(radix_scratch_ints(n));
+    ACHK(place(scratch, kRowShare, {{&d_key, n}, {&d_key2, n}, {&d_val2, n}, {&d_scr, scr + 64}}));
+    int* d_nlevs = d_scr + scr;
 
     // 0. validation (the status block must be clean before the bounded waits)
     {
@@ -532,11 +555,9 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
     const long long K = 7LL * nlevs;
 
     // 2-3. keys, counts, stable sort
-    ACHK(dalloc(&rec->slab[1], part(K + 1) + 2 * part((long long)nlevs + 1) + 64));
-    rec->d_counts = rec->slab[1];
-    int* d_levsz = rec->d_counts + part(K + 1);
-    rec->d_lptr = d_levsz + part((long long)nlevs + 1);
-    int* d_stats = rec->d_lptr + part((long long)nlevs + 1);
+    int *d_levsz, *d_stats;
+    ACHK(place(rec->slab, kOtherShare,
+               {{&rec->d_counts, K + 1}, {&d_levsz, nlevs + 1LL}, {&rec->d_lptr, nlevs + 1LL}, {&d_stats, 64}}));
     ACHK(cudaMemsetAsync(rec->d_counts, 0, sizeof(int) * (size_t)(K + 1), s));
     ACHK(cudaMemsetAsync(d_stats, 0, sizeof(rec->stats), s));
     if (n > 0) {
@@ -551,13 +572,18 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
 
     // 4. multirow warp map (always built; exposed in info for MULTIROW/ALL),
     // its scratch where the sort's keys were unless there are more keys than rows
-    const long long map_scr = 2 * part(K + 1) + part(scan_scratch_ints(K + 1));
-    if (map_scr > keys) {
-        cudaFree(scratch);
-        scratch = nullptr;
-        ACHK(dalloc(&scratch, map_scr));
+    int *d_wpk = d_key, *d_rowoff = d_key2, *d_scr2 = d_val2;
+    bool fits = K + 1 <= n;
+    if (scratch.size() == 1) {  // the three arrays are one stretch
+        const long long pk = block_part(K + 1);
+        fits = 2 * pk + block_part(scan_scratch_ints(K + 1)) <= 3 * block_part(n);
+        d_rowoff = d_wpk + pk;
+        d_scr2 = d_rowoff + pk;
     }
-    int *d_wpk = scratch, *d_rowoff = d_wpk + part(K + 1), *d_scr2 = d_rowoff + part(K + 1);
+    if (!fits) {
+        free_blocks(scratch);
+        ACHK(place(scratch, kOtherShare, {{&d_wpk, K + 1}, {&d_rowoff, K + 1}, {&d_scr2, scan_scratch_ints(K + 1)}}));
+    }
     int n_warps = 0;
     if (K > 0) {
         k_warps_per_key<<<grid_for(K + 1, 256), 256, 0, s>>>(rec->d_counts, (int)K, d_wpk);
@@ -572,11 +598,7 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
         ACHK(cudaStreamSynchronize(s));
     }
     rec->n_warps = n_warps;
-    const long long pw = part((long long)n_warps + 1);
-    ACHK(dalloc(&rec->slab[2], 3 * pw));
-    rec->d_ibase = rec->slab[2];
-    rec->d_ivect = rec->d_ibase + pw;
-    rec->d_wlev = rec->d_ivect + pw;
+    ACHK(place(rec->slab, kOtherShare, {{&rec->d_ibase, n_warps + 1LL}, {&rec->d_ivect, n_warps}, {&rec->d_wlev, n_warps}}));
     if (n_warps > 0) {
         k_warp_map<<<grid_for(n_warps, 256), 256, 0, s>>>(d_wpk, d_rowoff, (int)K, n_warps, n, rec->d_ibase,
                                                            rec->d_ivect, rec->d_wlev);
@@ -591,7 +613,7 @@ int run_analysis_impl(dfr_analysis_info_t* info, const sp_mat_t* L, MODE mode, c
         ACHK(cudaGetLastError());
     }
     ACHK(cudaStreamSynchronize(s));
-    cudaFree(scratch);
+    free_blocks(scratch);
 #undef ACHK
 
     info->mode = mode;

@@ -11,6 +11,7 @@
 #include <stdexcept>
 #include <system_error>
 #include <unordered_map>
+#include <vector>
 
 #include "common.cuh"
 #include "sptrsv_b200.h"
@@ -199,11 +200,16 @@ struct AnalysisRec {
     int* d_wlev = nullptr;     // [n_warps]
     int* d_lptr = nullptr;     // [nlevs+1] first iorder position of each level
     int stats[20] = {};        // level widths and row lengths (k_level_sizes), grid lines (k_line_check)
-    int* slab[5] = {};         // the allocations that hold these arrays and the info struct's
+    std::vector<int*> slab;    // the allocations that hold these arrays and the info struct's
     bool map_in_info = false;  // map arrays are also referenced by the info struct
     int* tile_tasks[6] = {};   // level-aligned iorder tasks for 32>>j lanes per row
     int tile_ntasks[6] = {};
 };
+inline void free_blocks(std::vector<int*>& blocks)
+{
+    for (int* q : blocks) cudaFree(q);
+    blocks.clear();
+}
 // How one CTA would take a system level by level (level_cta.cuh): kp lanes per
 // row, teams of g warps; kp = 0: the sync-free kernels are the faster ones.
 struct LevelCtaShape {

@@ -308,7 +308,7 @@ void free_device_analysis(sp_mat_t* gpu_L, dfr_analysis_info_t* info)
         if (info) {
             AnalysisRec* rec = info->row_ctr ? unregister_analysis(info->row_ctr) : nullptr;
             if (rec) {
-                for (int* q : rec->slab) cudaFree(q);  // every array of info is part of one of them
+                free_blocks(rec->slab);  // every array of info is part of one of them
                 for (int j = 0; j < 6; j++) cudaFree(rec->tile_tasks[j]);
                 delete rec;
             } else {
