@@ -215,7 +215,7 @@ void band_spread(int n, F&& f)
 
 void band_free(BandLayout& t)
 {
-    cudaFree(t.rec64); cudaFree(t.rec32); cudaFree(t.ustep);
+    cudaFree(t.rec64); cudaFree(t.rec32); cudaFree(t.ustep); cudaFree(t.own_b);
     t = BandLayout{};
 }
 
@@ -347,7 +347,8 @@ int build_band_layout(sptrsv_plan_s* p)
         return code;
     };
     if (dalloc(&t.ustep, nunits + 1) != cudaSuccess || dalloc(&t.rec64, (long long)ns * rb64) != cudaSuccess ||
-        dalloc(&t.rec32, (long long)ns * rb32) != cudaSuccess)
+        dalloc(&t.rec32, (long long)ns * rb32) != cudaSuccess ||
+        (!p->part_tab.empty() && dalloc(&t.own_b, p->part_tab[p->part_tab.size() - 2]) != cudaSuccess))
         return fail(cuda_fail(cudaGetLastError(), "band layout"));
     if (cudaMemcpy(t.ustep, ustep.data(), sizeof(int) * (size_t)(nunits + 1), cudaMemcpyHostToDevice) != cudaSuccess ||
         (ns > 0 && (cudaMemcpy(t.rec64, h64.data(), h64.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -368,19 +369,20 @@ int band_solve(sptrsv_plan_s* p, bool f32, const void* b, bool b_f32, void* x, d
     if (t.nsteps == 0) return 0;
     const double* bd = static_cast<const double*>(b);
     const float* bf = static_cast<const float*>(b);
-    if (!f32) {
-        double* xd = static_cast<double*>(x);
-        if (!p->part_tab.empty()) {
-            // warm-up rows read b of rows that another unit writes x of: a solve in place takes a copy of b
-            const long long m = p->part_tab[p->part_tab.size() - 2];  // end of the last block
-            if (xd < bd + m && bd < xd + m) {
-                if (!p->band_b) SPT_CUDA(dalloc(&p->band_b, m));
-                SPT_CUDA(cudaMemcpyAsync(p->band_b, bd, sizeof(double) * (size_t)m, cudaMemcpyDeviceToDevice, s));
-                bd = p->band_b;
-            }
+    if (t.own_b) {
+        // warm-up rows read b of rows that another unit writes the result of: a solve in place takes a copy of b
+        const size_t m = (size_t)p->part_tab[p->part_tab.size() - 2];  // end of the last block
+        const size_t bytes = m * (b_f32 ? sizeof(float) : sizeof(double));
+        auto overlaps = [&](const void* y, size_t elem) {
+            return y && (uintptr_t)y < (uintptr_t)b + bytes && (uintptr_t)b < (uintptr_t)y + m * elem;
+        };
+        if (overlaps(x, f32 ? sizeof(float) : sizeof(double)) || overlaps(x64, sizeof(double))) {
+            SPT_CUDA(cudaMemcpyAsync(t.own_b, b, bytes, cudaMemcpyDeviceToDevice, s));
+            bd = t.own_b;
+            bf = reinterpret_cast<const float*>(t.own_b);
         }
-        return band_launch_t<double, double, OUT_X>(t, t.rec64, bd, xd, nullptr, s);
     }
+    if (!f32) return band_launch_t<double, double, OUT_X>(t, t.rec64, bd, static_cast<double*>(x), nullptr, s);
     float* xf = static_cast<float*>(x);
     if (out_mode == OUT_SET64)
         return b_f32 ? band_launch_t<float, float, OUT_SET64>(t, t.rec32, bf, xf, x64, s)

@@ -96,6 +96,7 @@ struct Wave4Layout {
     int ngroups = 0, G = 0;
     int places = 0;            // most of one group in shared memory
     double* xp = nullptr;      // [npub] the chunks that another group reads (FP32 solves: as floats)
+    double* own_b = nullptr;   // [rows of the outer plan] b of a solve in place
     int npub = 0;
 };
 
@@ -121,6 +122,7 @@ struct BandLayout {
     int* ustep = nullptr;      // [nunits+1] first step of each unit
     unsigned char* rec64 = nullptr;  // [nsteps * rb64]
     unsigned char* rec32 = nullptr;  // [nsteps * rb32]
+    double* own_b = nullptr;   // block systems only: [rows of the outer plan] b of a solve in place
     int rb64 = 0, rb32 = 0;
 };
 
@@ -203,7 +205,6 @@ struct sptrsv_plan_s {
     // plan's rows directly
     std::vector<int> part_tab;
     BandLayout band;             // BAND layout (built on demand)
-    double* band_b = nullptr;    // block systems only: b of a solve in place (built on demand)
 };
 
 namespace sptrsv {

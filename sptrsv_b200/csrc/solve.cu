@@ -311,7 +311,6 @@ void plan_free_arrays(sptrsv_plan_s* p)
     cudaFree(p->bflag);
     part_free(p);
     band_free(p->band);
-    cudaFree(p->band_b);
     if (p->epochs) cudaFreeHost(p->epochs);
     if (p->ev_start) cudaEventDestroy(p->ev_start);
     if (p->ev_copied) cudaEventDestroy(p->ev_copied);
@@ -722,11 +721,7 @@ int part_own_rhs(sptrsv_plan_s* p, const BT* b, const X* x, cudaStream_t s, cons
     const uintptr_t b0 = (uintptr_t)b, x0 = (uintptr_t)x, m = (uintptr_t)p->n;
     *out = b;
     if (!x || x0 >= b0 + m * sizeof(BT) || b0 >= x0 + m * sizeof(X)) return 0;
-    int e = part_ensure(p->part, 1);
-    if (e) return e;
-    BT* copy;
-    if constexpr (sizeof(BT) == 8) copy = p->part->bx;
-    else copy = p->part->bx32;
+    BT* copy = reinterpret_cast<BT*>(p->part->sub->wave4.own_b);
     SPT_CUDA(cudaMemcpyAsync(copy, b, sizeof(BT) * (size_t)m, cudaMemcpyDeviceToDevice, s));
     *out = copy;
     return 0;

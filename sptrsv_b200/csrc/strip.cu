@@ -196,7 +196,7 @@ void wave4_free(Wave4Layout& w)
 {
     cudaFree(w.inv64); cudaFree(w.inv32); cudaFree(w.lsub64); cudaFree(w.lsub32); cudaFree(w.ev64); cudaFree(w.ev32);
     cudaFree(w.ecol); cudaFree(w.chunk); cudaFree(w.runc); cudaFree(w.grun); cudaFree(w.grow); cudaFree(w.gseq);
-    cudaFree(w.gmap); cudaFree(w.xp);
+    cudaFree(w.gmap); cudaFree(w.xp); cudaFree(w.own_b);
     w = Wave4Layout{};
 }
 
@@ -390,6 +390,7 @@ int build_wave4(sptrsv_plan_s* p, int G, int max_rows)
         if (pub[q]) w.npub += (hchunk[4 * (size_t)q + 1] + Q - 1) / Q * Q;
     }
     W4CHK(dalloc(&w.xp, std::max(1, w.npub)));
+    W4CHK(dalloc(&w.own_b, p->part_tab[p->part_tab.size() - 2]));  // here: a solve may be captured
     const long long ns = (long long)nch * C;
     W4CHK(dalloc(&w.inv64, ns));
     W4CHK(dalloc(&w.inv32, ns));
