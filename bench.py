@@ -475,14 +475,23 @@ def chain_hop_us(torch, S, SEL, n=100_000):
     return out
 
 
-def load_traffic(kernel_key: str):
+def load_traffic(kernel_key: str, schedule: str | None = None):
+    """DRAM bytes a launch of the solve kernel moves, from the capture on record;
+    with a schedule, only when the capture is of that very one."""
     p = ROOT / "profiles" / "ncu_traffic.json"
     if p.exists():
-        d = json.loads(p.read_text())
-        v = d.get(kernel_key)
-        if isinstance(v, dict):
+        v = json.loads(p.read_text()).get(kernel_key)
+        if isinstance(v, dict) and (schedule is None or schedule in v.get("schedules", [])):
             return v.get("dram_bytes_per_launch")
     return None
+
+
+def one_coupling(m) -> bool:
+    """Does every row read at most one row besides the one before it (a 2D
+    five-point stencil)?"""
+    rows = np.repeat(np.arange(m.n), np.diff(m.rowptr))
+    outside = rows[m.colidx < rows - 1]
+    return outside.size == 0 or int(np.bincount(outside).max()) <= 1
 
 
 def run_ours(args, rank, world, local, dist):
@@ -587,7 +596,7 @@ def run_ours(args, rank, world, local, dist):
     ms_per_step = total_ms / args.steps
     picked = SEL.schedule_from_class(sel64 if mode == 64 else sel32)
     launches_per_step = solve_launches(picked, mode, ir_iters, k == 1 and (
-        picked.variant == 6 or (picked.variant == 5 and args.config == "c1")))
+        picked.variant == 6 or (picked.variant == 5 and one_coupling(m))))
 
     # --- the other mode and the drop-in FP64 path
     other = 32 if mode == 64 else 64
@@ -618,7 +627,8 @@ def run_ours(args, rank, world, local, dist):
     variant = SEL.VARIANT_NAMES[sched.variant]
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": load_traffic(f"{variant}{f'_p{sched.partitions}' if sched.partitions >= 2 else ''}"
-                                        f"_{'f64' if mode == 64 else 'f32'}_{args.config}"),
+                                        f"_{'f64' if mode == 64 else 'f32'}_{args.config}",
+                                        SEL.class_name(sel64 if mode == 64 else sel32)),
                 "kernel": kname, "algorithmic_bytes_per_launch": bytes_kern, "launch_ms": t_kern,
                 "peak_kind": peak_kind}
     if not args.extra:
@@ -838,7 +848,8 @@ def run_batch(args, rank, world, local, dist):
     apply(best)
     achieved = nbytes / (t64 / 1e3) / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": load_traffic(f"batch{f'_p{c64[0]}' if c64[0] else ''}_f64_c3"),
+                "traffic": load_traffic(f"batch{f'_p{c64[0]}' if c64[0] else ''}_f64_c3",
+                                        f"mode{c64[1]}-width{c64[2]:g}-bw{c64[3]}"),
                 "kernel": "k_sptrsv_vk (one FP64 launch per solve)",
                 "algorithmic_bytes_per_launch": nbytes, "launch_ms": t64, "peak_kind": peak_kind,
                 "union_levels": batch.nlevs}
