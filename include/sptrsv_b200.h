@@ -188,7 +188,9 @@ int sptrsv_analysis_buckets(const dfr_analysis_info_t* info, int* host_buckets);
 
 /* Order-coop variant (solver/solve_csr_order.cu:11-77, disabled in the
  * reference by ORDER_COOP 0): iorder sequence, `tile` lanes per row
- * (tile in {1,2,4,8,16,32}).  b, x DEVICE arrays. */
+ * (tile in {1,2,4,8,16,32}).  b, x DEVICE arrays.  Where few rows a level or
+ * lines of a stencil let the ORDER and MULTIROW solves take another kernel, this
+ * one takes it too, and tile has no bearing. */
 int sptrsv_solve_order_tile(sp_mat_t* mat, dfr_analysis_info_t* info, const double* b,
                             double* x, int tile, cudaStream_t stream);
 
@@ -223,10 +225,13 @@ typedef struct {
     int variant;          /* SPTRSV_VAR_*                                            */
     int rows_per_warp;    /* 1,2,4,8,16,32: lanes per row = 32/rows_per_warp         */
                           /* (MULTIROW takes lanes per row from the analysis map;     */
-                          /* STRIP: chunk runs per warp)                              */
+                          /* STRIP: chunk runs per warp; SIMPLE and BAND: no bearing) */
     int block_warps;      /* warps per CTA: 2, 4, 8 or 16                             */
     int warps_per_sm;     /* resident warps per SM of the persistent grid (0 = max)   */
     int backoff_ns;       /* nanosleep between polls after 8 failed polls (0 = spin)  */
+                          /* (ORDER and MULTIROW with one right-hand side on levels   */
+                          /* of few rows: one CTA solves them, and rows_per_warp,     */
+                          /* block_warps, warps_per_sm and backoff_ns have no bearing)*/
     int ir_max_iters;     /* FP32+IR: refinement steps after the first FP32 solve     */
     int band_levels;      /* CLUSTER: levels per band (H)                             */
     int cluster_rows;     /* CLUSTER: rows per cluster (B, <= 8192)                   */

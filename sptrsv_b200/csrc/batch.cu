@@ -14,7 +14,7 @@
 // A system whose levels hold few rows on average (n_s / nlevs_s below a
 // threshold; a near-chain) gains nothing from the level order: every level
 // costs a cross-warp hop through L2.  The hybrid schedule gives each such
-// system to a team of up to four warps of the same persistent launch, which
+// system to a team of up to seven warps of the same persistent launch, which
 // walks it in natural order, the rows handed on from warp to warp by named
 // barriers and the recent x values in a shared-memory ring (seq_unit).  The
 // other systems keep the level-ordered tasks on the remaining warps.
